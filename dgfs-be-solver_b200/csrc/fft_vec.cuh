@@ -1,0 +1,232 @@
+// Register-resident complex FFTs of compile-time length, natural order in and
+// out, with the conventions of fft_reg.cuh:
+//
+//   cfft<N, S>(x):  x[k] <- sum_n x[n] exp(S 2 pi i n k / N)
+//
+// Two element types: double2, and cpx, an FP32 complex number in one 64-bit
+// register pair.  On cpx one packed instruction (add/sub/mul/fma.rn.f32x2)
+// works on the real and the imaginary part together.  The packed instructions
+// run at the FP32 pipe's rate (128 lanes per clock and SM, the same as scalar
+// ones: measured), so they take half the issue slots, which is what the
+// transforms of the collision kernels were short of.  Where a value is needed
+// times i, its producer writes the parts in swapped order with two scalar
+// adds (the same pipe time as one packed add) and the consumer is an FMA
+// with (-1, 1) factors.
+//
+// N = 2^m is a decimation in time down to 8-point kernels whose sqrt(1/2)
+// factors are folded into FMAs (52 operations).  N = 24 is the prime-factor
+// (Good-Thomas) transform: 3 and 8 have no common factor, so 8 three-point
+// and 3 eight-point transforms need no twiddle factors between them (252
+// operations against 308 for the mixed-radix 8 x 3 transform of fft_reg.cuh);
+// its index maps are compile-time register names.
+#pragma once
+
+#include "dgfs_common.cuh"
+
+namespace dgfs {
+
+struct cpx {
+  unsigned long long v;  // low half: real part
+};
+
+__device__ __forceinline__ cpx cpk(float re, float im) {
+  cpx r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(re), "f"(im));
+  return r;
+}
+__device__ __forceinline__ float cre(cpx a) { return __uint_as_float((unsigned)a.v); }
+__device__ __forceinline__ float cim(cpx a) { return __uint_as_float((unsigned)(a.v >> 32)); }
+// the element type of a precision, from and to its parts and to float2 / double2
+template <typename T> struct vec_of;
+template <> struct vec_of<float> { using type = cpx; };
+template <> struct vec_of<double> { using type = double2; };
+template <typename T> using vx = typename vec_of<T>::type;
+__device__ __forceinline__ cpx vmk(float re, float im) { return cpk(re, im); }
+__device__ __forceinline__ double2 vmk(double re, double im) { return make_double2(re, im); }
+__device__ __forceinline__ double cre(double2 a) { return a.x; }
+__device__ __forceinline__ double cim(double2 a) { return a.y; }
+__device__ __forceinline__ cpx from_c(float2 a) { return cpk(a.x, a.y); }
+__device__ __forceinline__ double2 from_c(double2 a) { return a; }
+__device__ __forceinline__ float2 to_c(cpx a) { return make_float2(cre(a), cim(a)); }
+__device__ __forceinline__ double2 to_c(double2 a) { return a; }
+
+__device__ __forceinline__ cpx vadd(cpx a, cpx b) {
+  cpx r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ cpx vsub(cpx a, cpx b) {
+  cpx r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ cpx vmul(cpx a, cpx b) {  // part by part
+  cpx r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ cpx vfma(cpx a, cpx b, cpx c) {  // a b + c part by part
+  cpx r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ double2 vmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+
+// a + i s h b from bs = b with its parts swapped: (a.x - s h b.y, a.y + s h b.x);
+// S = +-1, H = 0 (h = 1) or 1 (h = sin(pi/3))
+template <int S, int H> __device__ __forceinline__ cpx add_rot(cpx a, cpx bs) {
+  constexpr float h = H ? 0.86602540378443864676f : 1.f;
+  return vfma(bs, cpk(-S * h, S * h), a);
+}
+template <int S, int H> __device__ __forceinline__ double2 add_rot(double2 a, double2 bs) {
+  if constexpr (H) return make_double2(fma(bs.x, -S * 0.86602540378443864676, a.x), fma(bs.y, S * 0.86602540378443864676, a.y));
+  else if constexpr (S > 0) return make_double2(a.x - bs.x, a.y + bs.y);
+  else return make_double2(a.x + bs.x, a.y - bs.y);
+}
+// a - b with the parts swapped
+__device__ __forceinline__ cpx sub_swap(cpx a, cpx b) { return cpk(cim(a) - cim(b), cre(a) - cre(b)); }
+__device__ __forceinline__ double2 sub_swap(double2 a, double2 b) { return make_double2(a.y - b.y, a.x - b.x); }
+// (1 + i S) a
+template <int S> __device__ __forceinline__ cpx mul_1i(cpx a) {
+  return S > 0 ? cpk(cre(a) - cim(a), cim(a) + cre(a)) : cpk(cre(a) + cim(a), cim(a) - cre(a));
+}
+template <int S> __device__ __forceinline__ double2 mul_1i(double2 a) {
+  return S > 0 ? make_double2(a.x - a.y, a.y + a.x) : make_double2(a.x + a.y, a.y - a.x);
+}
+// a + S sqrt(1/2) t
+template <int S> __device__ __forceinline__ cpx add_h(cpx a, cpx t) {
+  return vfma(t, cpk(S * 0.70710678118654752440f, S * 0.70710678118654752440f), a);
+}
+template <int S> __device__ __forceinline__ double2 add_h(double2 a, double2 t) {
+  return make_double2(fma(t.x, S * 0.70710678118654752440, a.x), fma(t.y, S * 0.70710678118654752440, a.y));
+}
+// a - b / 2
+__device__ __forceinline__ cpx sub_half(cpx a, cpx b) { return vfma(b, cpk(-0.5f, -0.5f), a); }
+__device__ __forceinline__ double2 sub_half(double2 a, double2 b) {
+  return make_double2(fma(b.x, -0.5, a.x), fma(b.y, -0.5, a.y));
+}
+// a + i S b
+template <int S> __device__ __forceinline__ cpx add_i(cpx a, cpx b) {
+  return S > 0 ? cpk(cre(a) - cim(b), cim(a) + cre(b)) : cpk(cre(a) + cim(b), cim(a) - cre(b));
+}
+template <int S> __device__ __forceinline__ double2 add_i(double2 a, double2 b) {
+  return S > 0 ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, a.y - b.x);
+}
+// a (c + i s)
+__device__ __forceinline__ cpx mul_w(cpx a, double c, double s) {
+  const float wc = (float)c, ws = (float)s;
+  return cpk(fmaf(-ws, cim(a), wc * cre(a)), fmaf(ws, cre(a), wc * cim(a)));
+}
+__device__ __forceinline__ double2 mul_w(double2 a, double c, double s) {
+  return make_double2(fma(-s, a.y, c * a.x), fma(s, a.x, c * a.y));
+}
+
+// cos(2 pi j / 32), j <= 8
+__host__ __device__ constexpr double cos32(int j) {
+  return j == 0 ? 1.0
+       : j == 1 ? 0.98078528040323044913
+       : j == 2 ? 0.92387953251128675613
+       : j == 3 ? 0.83146961230254523708
+       : j == 4 ? 0.70710678118654752440
+       : j == 5 ? 0.55557023301960222474
+       : j == 6 ? 0.38268343236508977173
+       : j == 7 ? 0.19509032201612826785
+                : 0.0;
+}
+// cos and sin of 2 pi j / N (N divides 32), j < N / 2
+template <int N> __host__ __device__ constexpr double tcos(int j) {
+  return j * (32 / N) <= 8 ? cos32(j * (32 / N)) : -cos32(16 - j * (32 / N));
+}
+template <int N> __host__ __device__ constexpr double tsin(int j) {
+  return j * (32 / N) <= 8 ? cos32(8 - j * (32 / N)) : cos32(j * (32 / N) - 8);
+}
+
+// SW: the third output with its parts swapped
+template <int S, bool SW, typename C> __device__ __forceinline__ void cfft4(C& a, C& b, C& c, C& d) {
+  const C s0 = vadd(a, c), d0 = vsub(a, c), s1 = vadd(b, d), d1 = sub_swap(b, d);
+  a = vadd(s0, s1);
+  if constexpr (SW) c = sub_swap(s0, s1);
+  else c = vsub(s0, s1);
+  b = add_rot<S, 0>(d0, d1);
+  d = add_rot<-S, 0>(d0, d1);
+}
+
+// 8 points, outputs x0 .. x7 in place of inputs x0 .. x7
+template <int S, typename C>
+__device__ __forceinline__ void cfft8(C& x0, C& x1, C& x2, C& x3, C& x4, C& x5, C& x6, C& x7) {
+  C e0 = x0, e1 = x2, e2 = x4, e3 = x6, o0 = x1, o1 = x3, o2 = x5, o3 = x7;
+  cfft4<S, false>(e0, e1, e2, e3);
+  cfft4<S, true>(o0, o1, o2, o3);
+  x0 = vadd(e0, o0);
+  x4 = vsub(e0, o0);
+  const C t1 = mul_1i<S>(o1), t3 = mul_1i<-S>(o3);
+  x1 = add_h<1>(e1, t1);
+  x5 = add_h<-1>(e1, t1);
+  x2 = add_rot<S, 0>(e2, o2);
+  x6 = add_rot<-S, 0>(e2, o2);
+  x3 = add_h<-1>(e3, t3);
+  x7 = add_h<1>(e3, t3);
+}
+
+template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[N]) {
+  if constexpr (N == 4) {
+    cfft4<S, false>(x[0], x[1], x[2], x[3]);
+  } else if constexpr (N == 8) {
+    cfft8<S>(x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]);
+  } else if constexpr (N == 24) {
+    // n = 8 n1 + 3 n2, k = 16 k1 + 9 k2 (mod 24): W24^{nk} = W3^{n1 k1} W8^{n2 k2}
+    sfor<0, 8>([&](auto c) {
+      constexpr int n = 3 * decltype(c)::value;
+      C &a = x[n % 24], &b = x[(8 + n) % 24], &d = x[(16 + n) % 24];
+      const C s = vadd(b, d), ds = sub_swap(b, d), e = sub_half(a, s);
+      a = vadd(a, s);
+      b = add_rot<S, 1>(e, ds);
+      d = add_rot<-S, 1>(e, ds);
+    });
+    C y[24];
+    sfor<0, 3>([&](auto c) {
+      constexpr int m = 8 * decltype(c)::value, q = 16 * decltype(c)::value;
+      C t[8];
+      sfor<0, 8>([&](auto i) { t[decltype(i)::value] = x[(m + 3 * decltype(i)::value) % 24]; });
+      cfft8<S>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7]);
+      sfor<0, 8>([&](auto i) { y[(q + 9 * decltype(i)::value) % 24] = t[decltype(i)::value]; });
+    });
+#pragma unroll
+    for (int i = 0; i < 24; ++i) x[i] = y[i];
+  } else {
+    C e[N / 2], o[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      e[i] = x[2 * i];
+      o[i] = x[2 * i + 1];
+    }
+    cfft<N / 2, S>(e);
+    cfft<N / 2, S>(o);
+    sfor<0, N / 2>([&](auto c) {
+      constexpr int j = decltype(c)::value;
+      if constexpr (8 * j == N) {
+        const C t = mul_1i<S>(o[j]);
+        x[j] = add_h<1>(e[j], t);
+        x[j + N / 2] = add_h<-1>(e[j], t);
+      } else if constexpr (8 * j == 3 * N) {
+        const C t = mul_1i<-S>(o[j]);
+        x[j] = add_h<-1>(e[j], t);
+        x[j + N / 2] = add_h<1>(e[j], t);
+      } else if constexpr (4 * j == N) {
+        x[j] = add_i<S>(e[j], o[j]);
+        x[j + N / 2] = add_i<-S>(e[j], o[j]);
+      } else {
+        const C t = j == 0 ? o[j] : mul_w(o[j], tcos<N>(j), S * tsin<N>(j));
+        x[j] = vadd(e[j], t);
+        x[j + N / 2] = vsub(e[j], t);
+      }
+    });
+  }
+}
+
+}  // namespace dgfs

@@ -115,4 +115,59 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float(r);
 }
 
+// Tensor memory as a warp's scratchpad: each thread owns one lane (the warp's
+// quarter, 32 (warp % 4) + lane) and any columns, 32 bits each.  A load's
+// registers hold its values after tmem_wait on them, which waits for every
+// load of the thread; tmem_store_wait completes the thread's stores.
+__device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]) : : "memory");
+}
+__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
+__device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) : : "memory");
+}
+__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// n consecutive columns (a multiple of 8) of this thread's lane
+template <int n> __device__ __forceinline__ void tm_load(uint32_t col, uint32_t (&t)[n]) {
+  static_assert(n % 8 == 0, "columns in steps of 8");
+#pragma unroll
+  for (int c = 0; c + 16 <= n; c += 16) tmem_load(col + c, *reinterpret_cast<uint32_t(*)[16]>(&t[c]));
+  if constexpr (n % 16) tmem_load(col + n / 16 * 16, *reinterpret_cast<uint32_t(*)[8]>(&t[n / 16 * 16]));
+}
+template <int n> __device__ __forceinline__ void tm_wait(uint32_t (&t)[n]) {
+#pragma unroll
+  for (int c = 0; c + 16 <= n; c += 16) tmem_wait(*reinterpret_cast<uint32_t(*)[16]>(&t[c]));
+  if constexpr (n % 16) tmem_wait(*reinterpret_cast<uint32_t(*)[8]>(&t[n / 16 * 16]));
+}
+template <int n> __device__ __forceinline__ void tm_store(uint32_t col, const uint32_t (&t)[n]) {
+#pragma unroll
+  for (int c = 0; c + 16 <= n; c += 16) tmem_store(col + c, *reinterpret_cast<const uint32_t(*)[16]>(&t[c]));
+  if constexpr (n % 16) tmem_store(col + n / 16 * 16, *reinterpret_cast<const uint32_t(*)[8]>(&t[n / 16 * 16]));
+}
+// a real value as words of tensor memory (1 or 2), at compile-time position i
+template <int n> __device__ __forceinline__ void tm_put(uint32_t (&t)[n], int i, float v) { t[i] = __float_as_uint(v); }
+template <int n> __device__ __forceinline__ void tm_put(uint32_t (&t)[n], int i, double v) {
+  t[2 * i] = (uint32_t)__double2loint(v);
+  t[2 * i + 1] = (uint32_t)__double2hiint(v);
+}
+template <int n> __device__ __forceinline__ float tm_get(const uint32_t (&t)[n], int i, float) {
+  return __uint_as_float(t[i]);
+}
+template <int n> __device__ __forceinline__ double tm_get(const uint32_t (&t)[n], int i, double) {
+  return __hiloint2double((int)t[2 * i + 1], (int)t[2 * i]);
+}
+
 }  // namespace dgfs

@@ -13,8 +13,8 @@
 #include "../../include/dgfs_b200.h"
 #include "dgfs_internal.h"
 #include "vhs_push.cuh"
-#include "vhs_cube.cuh"
 #include "vhs_pair.cuh"
+#include "vhs_variant.h"
 
 namespace dgfs {
 
@@ -47,15 +47,6 @@ static int init_twiddles(int dev) {
 // ---------------------------------------------------------------------------
 // Kernel variants
 // ---------------------------------------------------------------------------
-struct VhsVariant {
-  int prec, N, C, db, minb, threads, push;
-  size_t smem;
-  size_t scratch_cx;  // two-CTA kernel: complex scratch per cluster
-  const void* fn;
-  cudaError_t (*launch32)(const VhsArgs<float>&, int, cudaStream_t);
-  cudaError_t (*launch64)(const VhsArgs<double>&, int, cudaStream_t);
-};
-
 template <typename T, int N, int C, bool DB, int MINB>
 static cudaError_t launch_vhs(const VhsArgs<T>& a, int nclusters, cudaStream_t s) {
   using G = VhsGeom<N, C, DB>;
@@ -125,42 +116,6 @@ template <typename T, int N, int C, int MINB> static VhsVariant make_push() {
   return v;
 }
 
-template <int N, bool IL1> static cudaError_t launch_cube(const VhsArgs<float>& a, int nctas, cudaStream_t s) {
-  using G = CubeGeom<N>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nctas, 1, 1);
-  cfg.blockDim = dim3(G::NT, 1, 1);
-  cfg.dynamicSmemBytes = G::SMEM_CX * sizeof(cx<float>);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, vhs_cube_kernel<N, IL1>, a);
-}
-
-// single-CTA kernel (FP32; kind 2 in dgfs_vhs_variant_kind); IL1: the
-// first pass of every (p, q) transforms a thread's two lines together
-// (more ILP, more registers; db reports it)
-template <int N, bool IL1> static VhsVariant make_cube() {
-  using G = CubeGeom<N>;
-  VhsVariant v{};
-  v.prec = 32;
-  v.N = N;
-  v.C = 1;
-  v.db = IL1 ? 1 : 0;
-  v.push = 2;
-  v.minb = 1;
-  v.threads = G::NT;
-  v.smem = G::SMEM_CX * sizeof(cx<float>);
-  v.fn = (const void*)vhs_cube_kernel<N, IL1>;
-  v.launch32 = launch_cube<N, IL1>;
-  return v;
-}
-
 template <typename T, int N, int LPT>
 static cudaError_t launch_pair(const VhsArgs<T>& a, int nclusters, cudaStream_t s) {
   using G = PairGeom<T, N, LPT>;
@@ -201,25 +156,25 @@ template <typename T, int N, int LPT> static VhsVariant make_pair() {
 
 // Compiled launch shapes: (precision, N, cluster size, double-buffered
 // exchange, minimum CTAs per SM for the register budget).  The first entry
-// of each (precision, N) family is the default (FP32 N = 24: the single-CTA
-// kernel, 5.2 ms against 20 ms for the best cluster shape on 576 points;
-// FP64 N = 24 and FP32 N = 32: the two-CTA kernel, 15 ms against 50 ms and
-// 552 ms against 1,695 ms); the autotuner times the rest.
+// of each (precision, N) family is the default: the single-CTA kernel where a
+// point fits one SM (FP32 N = 24: 4.2 ms against 20 ms for the best cluster
+// shape on 576 points; FP32 N = 16: 0.49 ms against 1.16 ms on 592 points;
+// FP64 N = 16: 71 us against 204 us on one point), else the two-CTA kernel
+// (FP64 N = 24: 15 ms against 50 ms on 576 points; FP32 N = 32: 552 ms against
+// 1,695 ms on 10,368); the autotuner times the rest.
 static const std::vector<VhsVariant>& variants() {
   static const std::vector<VhsVariant> v = {
-      make_push<double, 8, 1, 4>(),             make_push<double, 16, 4, 2>(),
-      make_push<double, 16, 2, 1>(),            make_pair<double, 24, 1>(),
-      make_pair<double, 24, 2>(),               make_push<double, 24, 8, 1>(),
-      make_push<double, 24, 12, 1>(),           make_push<double, 32, 16, 1>(),
-      make_push<float, 8, 1, 4>(),              make_push<float, 16, 2, 2>(),
-      make_push<float, 16, 4, 4>(),             make_cube<24, false>(),
+      make_push<double, 8, 1, 4>(),             cube_variant(64, 16),
+      make_push<double, 16, 4, 2>(),            make_push<double, 16, 2, 1>(),
+      make_pair<double, 24, 1>(),               make_pair<double, 24, 2>(),
+      make_push<double, 24, 8, 1>(),            make_push<double, 24, 12, 1>(),
+      make_push<double, 32, 16, 1>(),           make_push<float, 8, 1, 4>(),
+      cube_variant(32, 16),                     make_push<float, 16, 2, 2>(),
+      make_push<float, 16, 4, 4>(),             cube_variant(32, 24),
       make_push<float, 24, 8, 2>(),             make_push<float, 24, 4, 1>(),
       make_push<float, 24, 12, 3>(),            make_pair<float, 32, 2>(),
-      make_pair<float, 32, 1>(),
-      make_push<float, 32, 16, 2>(),
-      make_push<float, 32, 8, 1>(),             make_cube<8, false>(),
-      make_cube<16, false>(),                   make_cube<16, true>(),
-      make_cube<24, true>(),
+      make_pair<float, 32, 1>(),                make_push<float, 32, 16, 2>(),
+      make_push<float, 32, 8, 1>(),             cube_variant(32, 8),
       make_variant<double, 8, 1, true, 4>(),    make_variant<double, 8, 2, true, 8>(),
       make_variant<double, 16, 4, true, 2>(),   make_variant<double, 16, 2, true, 1>(),
       make_variant<double, 16, 4, false, 3>(),
@@ -311,10 +266,10 @@ static int select_index(dgfs_vhs* h, int idx) {
   int ncl = 0, rc = variant_clusters(h, v, &ncl);
   if (rc) return rc;
   const size_t esz = h->prec == 64 ? 16 : 8;
-  // gain-spectrum scratch: one N^3 complex slice per cluster, or for the
-  // two-CTA kernel the half spectra of F and fC and the staging buffers
-  const size_t need = v->push == 3 ? (size_t)ncl * v->scratch_cx * esz
-                                   : (size_t)ncl * v->C * (size_t)h->N * h->N * h->N / v->C * esz;
+  // gain-spectrum scratch: one N^3 complex slice per cluster, one slice of the
+  // primary lines for the single-CTA kernel, or for the two-CTA kernel the
+  // half spectra of F and fC and the staging buffers
+  const size_t need = (size_t)ncl * (v->scratch_cx ? v->scratch_cx : (size_t)h->N * h->N * h->N) * esz;
   if (need > h->fc_bytes) {
     cudaFree(h->fc);
     h->fc = nullptr;
@@ -328,7 +283,7 @@ static int select_index(dgfs_vhs* h, int idx) {
     // kCubeSlices items per CTA, each with its own partial-spectrum slice,
     // and (at least 2 chunks per point) up to kCubeSlices / 2 points per CTA
     // with a chunk counter
-    const size_t needp = (size_t)kCubeSlices * ncl * (size_t)h->N * h->N * h->N * esz;
+    const size_t needp = (size_t)kCubeSlices * ncl * v->slice_cx * esz;
     if (needp > h->fcp_bytes) {
       cudaFree(h->fcp);
       h->fcp = nullptr;
@@ -680,6 +635,10 @@ static int vhs_launch(dgfs_vhs* h, const void* f, void* Q, int nupts, int neles,
     a.w1t = (const double*)h->w1t;
     a.b2t = (const double*)h->b2t;
     a.fc = (double2*)h->fc;
+    if (h->var->push == 2) {
+      a.fcp = (double2*)h->fcp;
+      a.pdone = h->pdone;
+    }
     a.err = h->err;
     a.plist = plist;
     a.pcount = pcount;

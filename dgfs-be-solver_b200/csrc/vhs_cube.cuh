@@ -1,4 +1,4 @@
-// Single-CTA fast-spectral VHS kernel for FP32 and N <= 24: the whole N^3
+// Single-CTA fast-spectral VHS kernel (FP32 N <= 24, FP64 N = 16): the whole N^3
 // problem of one point lives in one CTA's shared memory, so no transform
 // crosses SMs, and the transform count is nearly halved by an exact
 // restatement that uses the reality of f.
@@ -26,40 +26,77 @@
 // instead of two.  Per point: 1 + Nrho M + Nrho + 2 full transforms plus
 // the 2D ones (reference: 3 Nrho M + 3).
 //
-// Layout (shared memory, complex float): F for k3 <= N/2 ([N][N][N/2+1]),
-// the work cube as N^2 lines of N+1 (padding keeps line-parallel accesses
-// free of bank conflicts), the three Nyquist planes, the axis phases.
-// The gain spectrum fC accumulates in a global (L2-resident) slice per CTA,
-// stored with the last axis outermost so that the per-line accesses of a
-// warp are contiguous (w1 and b2 come in the same order, from their own
-// tables).
-// Main threads own two lines per pass; NQ extra threads (one line each)
-// transform the Nyquist planes during the first two passes of every (p, q).
+// One more restatement, also exact: with P = (1 + i) R, Re R^2 = Re P Im P
+// (and Re Nq^2 likewise), so the kernel transforms F^ = (1 + i) F and
+// accumulates one product per field.
+//
+// What bounds it: shared memory and the FP32 pipe, each about half busy, and
+// the passes' latencies.  Per (p, q) the work cube crosses shared memory four
+// times (two exchanges) and every complex value takes about 13 operations a
+// pass.  So: a thread owns one line (N = 24: 18 warps and 2 for the Nyquist
+// planes, five per scheduler; nine warps with two lines per thread left one
+// scheduler with half as many again as the others), in packed FP32 registers
+// (fft_vec.cuh: half the issue slots); everything that only its own thread
+// touches -- the spectrum line F^ and the sums S_p -- lives in tensor memory,
+// which costs neither registers nor shared-memory bandwidth (two lines per
+// thread with S_p in registers spilled: 5.7 ms a sweep, 4.7 ms with S_p in
+// tensor memory); and no shared access of the main threads conflicts.
+//
+// Layout in shared memory (complex float):
+//   sW   work cube: line (k1, k2) at k1 PS + off(k2), off(k) = N k + (k >= N/2).
+//        Half a warp of the first pass is 8 planes x {k2, k2 + N/2}, of the
+//        second 8 planes x {x3, x3 + 1}, of the third 8 x3 x {x2, x2 + N/2}:
+//        16 distinct 8-byte banks each (FP64: 8 lanes, 8 16-byte banks)
+//   sT1 [x2][x3], sT2 [x1][x3], sT3 [x2][x1]: the transformed Nyquist planes
+//   sN   [k][line] F^ on the Nyquist planes; sX their first axis
+//   phases of (p, q) and of the next, in two slots
+// The main threads are N/8 groups, each owning 8 planes k1: the second pass of
+// a group needs only that group's first pass, so groups synchronise among
+// themselves.  The third pass releases the cube as soon as its values are in
+// registers, so its arithmetic runs beside the next first pass.  NQ more
+// threads transform the Nyquist planes and fetch the next phases.  S_p is real, so the gain spectrum is kept for k1 <= N/2, in a global
+// (L2-resident) slice per CTA, [k3][line].
+//
+// Measured on one B200 (FP32, N = 24, 12 x 16 (p, q), 576 points): 4.16 ms a
+// sweep against 5.16 ms for the two-lines-per-thread kernel with scalar
+// transforms that this one replaces; FP32 pipe 48 % busy, shared memory 6.0K of
+// 9.9K cycles per (p, q).  N = 16 (8 x 6): 592 points 0.485 ms against 1.16 ms
+// for the two-CTA push kernel; FP64 N = 16, one point 71 us against 204 us
+// (its radial nodes spread over the SMs).
 #pragma once
 
+#include "fft_vec.cuh"
+#include "tcgen05.cuh"
 #include "vhs_kernel.cuh"
+#include "vhs_variant.h"
 
 namespace dgfs {
 
-template <int N> struct CubeGeom {
-  static constexpr int H = N / 2 + 1;
-  static constexpr int NN = N * N;
-  static constexpr int LP = N + 1;                      // padded line stride
-  static constexpr int NM = NN / 2;                     // main threads (2 lines)
-  static constexpr int NQ = ((3 * N + 31) / 32) * 32;  // Nyquist threads, one line each
+template <typename T, int N> struct CubeGeom {
+  static constexpr int HN = N / 2, H = HN + 1, NN = N * N, V = NN * N;
+  static constexpr int NM = NN;                      // main threads, one line each
+  static constexpr int GT = 8 * N;                   // threads per group of 8 planes
+  static constexpr int NQ = 3 * N <= 32 ? 32 : 64;   // Nyquist threads, one or two lines each
   static constexpr int NT = NM + NQ;
-  static constexpr int V = N * N * N;
-  static constexpr int PHS = 3 * N + 4;                 // one phase slot
-  // F at (k1, k2, k3 <= N/2) sits at k1 FS + k2 H + k3: one padding entry
-  // per k1 slab makes lanes that differ in k1 (the Nyquist-plane lines)
-  // fall in different banks
-  static constexpr int FS = N * H + 1;
-  static constexpr int OFF_F = 0;                       // [N][FS]
-  static constexpr int OFF_W = OFF_F + N * FS;          // [NN][LP]
-  static constexpr int OFF_T = OFF_W + NN * LP;         // [3][N][LP]
-  static constexpr int OFF_PH = OFF_T + 3 * N * LP;     // [2][PHS]
-  static constexpr int SMEM_CX = OFF_PH + 2 * PHS;
-  static_assert(NM % 32 == 0, "main threads must fill warps");
+  static constexpr int PS = NN + (sizeof(T) == 4 ? 2 : 1);  // plane stride of the work cube
+  static constexpr int PHS = 3 * N + 4;              // one phase slot
+  static constexpr int NL = H * N;                   // lines of the gain spectrum (k1 <= N/2)
+  static constexpr int SL = NL * N;                  // gain spectrum slice (complex)
+  // tensor memory columns: per main warp 2 N values of F^, then N of S
+  static constexpr int WD = sizeof(T) / 4;           // columns per value
+  static constexpr int TW = 3 * N * WD, TUSED = (NM / 32 + 3) / 4 * TW;
+  static constexpr int TCOLS = TUSED <= 32 ? 32 : TUSED <= 64 ? 64 : TUSED <= 128 ? 128 : TUSED <= 256 ? 256 : 512;
+  static constexpr int OFF_W = 0;
+  static constexpr int OFF_T1 = OFF_W + N * PS;
+  static constexpr int OFF_T2 = OFF_T1 + NN;
+  static constexpr int OFF_T3 = OFF_T2 + NN;
+  static constexpr int OFF_N = OFF_T3 + N * (N + 2);
+  static constexpr int OFF_X = OFF_N + 3 * NN;
+  static constexpr int OFF_PH = OFF_X + 3 * N * (N + 1);
+  static constexpr int SMEM = (OFF_PH + 2 * PHS) * 2 * (int)sizeof(T);  // bytes
+  __host__ __device__ static constexpr int off(int k) { return N * k + (k >= HN ? 1 : 0); }
+  static_assert(N % 8 == 0 && 3 * N <= 2 * NQ && NM % 32 == 0, "thread roles");
+  static_assert(OFF_T2 % 2 == 0 && OFF_T3 % 2 == 0 && OFF_PH % 2 == 0 && PHS % 2 == 0, "16-byte sections");
 };
 
 // Radial-node chunks per point.  A launch with few points would leave SMs
@@ -72,7 +109,6 @@ template <int N> struct CubeGeom {
 // capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch:
 // with P = 12 a split covers up to two waves of whole points).  Every CTA
 // computes the same value.
-constexpr int kCubeSlices = 24;
 __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
   if (P < 2 || (long long)npts * P > (long long)kCubeSlices * G) return 1;
   const double per_node = 3.0 * M + 3.0;
@@ -81,56 +117,83 @@ __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
   return split < whole ? P : 1;
 }
 
-template <int N, bool IL1>
-__global__ void __launch_bounds__(CubeGeom<N>::NT, 1) vhs_cube_kernel(const VhsArgs<float> a) {
-  using G = CubeGeom<N>;
-  using C = cx<float>;
-  constexpr int H = G::H, NN = G::NN, LP = G::LP, NM = G::NM, V = G::V, PHS = G::PHS, NT = G::NT, FS = G::FS;
-  constexpr int NY = N / 2;
+// Cycles between the starts of the second pass of a scheduler's successive
+// warps: staggered, the loads of one warp run beside the arithmetic of
+// another and the stores of a third (4.20 ms against 4.38 ms per 576 points
+// at N = 24 without; 60, 100 and 200 cycles measure the same).
+constexpr unsigned kStagger = 100;
+
+template <typename T, int N, int MINB>
+__global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(const VhsArgs<T> a) {
+  using G = CubeGeom<T, N>;
+  using C = vx<T>;   // in registers
+  using CM = cx<T>;  // in the tables and the scratch
+  constexpr int WD = G::WD;
+  constexpr int HN = G::HN, NN = G::NN, V = G::V, NM = G::NM, GT = G::GT, NT = G::NT, PS = G::PS, PHS = G::PHS;
+  constexpr int B_ALL = 0, B_T = 1, B_G = 2;  // named barriers: CTA, Nyquist tables, groups
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* const sF = reinterpret_cast<C*>(smem_raw) + G::OFF_F;
-  C* const sW = reinterpret_cast<C*>(smem_raw) + G::OFF_W;
-  C* const sT1 = reinterpret_cast<C*>(smem_raw) + G::OFF_T;
-  C* const sT2 = sT1 + N * LP;
-  C* const sT3 = sT2 + N * LP;
-  C* const sPh = reinterpret_cast<C*>(smem_raw) + G::OFF_PH;
+  C* const base = reinterpret_cast<C*>(smem_raw);
+  C* const sW = base + G::OFF_W;
+  C* const sT1 = base + G::OFF_T1;
+  C* const sT2 = base + G::OFF_T2;
+  C* const sT3 = base + G::OFF_T3;
+  C* const sN = base + G::OFF_N;
+  C* const sX = base + G::OFF_X;
+  CM* const sPh = reinterpret_cast<CM*>(base + G::OFF_PH);
   __shared__ double sRed[5][NT / 32];
   __shared__ double sLam[5];
+  __shared__ uint32_t s_tmem;
+  __shared__ __align__(8) uint64_t s_read;  // every main warp has read its part of the cube
+  __shared__ int s_gave_up;
 
   const int tid = threadIdx.x;
   const bool is_main = tid < NM;
   const int tq = tid - NM;
-  C* const fcg = a.fc + (size_t)blockIdx.x * V;
-  const float invV = 1.f / (float)V;
+  CM* const fcg = a.fc + (size_t)blockIdx.x * G::SL;
   const int npq = a.P * a.M;
 
-  // axis phases e^{i fac_p s_q[ax] l0[k]} of (p, q), and
-  // Theta_ax = e^{i fac_p N s_q[ax]} = conj(e^{i fac_p s_q[ax] l0[N/2]})^2.
-  // Threads tid < 3N each carry one entry: fetched from L2 at the start of
-  // a pass (phase_fetch), stored to the other slot at its end
-  // (phase_store), so the load latency hides behind the pass.
-  static_assert(3 * N <= NT, "one phase entry per thread");
-  auto phase_fetch = [&](int pq) -> C {
-    return tid < 3 * N ? a.phase[(size_t)pq * 3 * N + tid] : mk<C>(0.f, 0.f);
+  // roles of a main thread: first pass line (k1, k2), second pass line
+  // (k1, x3 = r), third pass line (x2 = r, x3 = k1)
+  const int grp = tid / GT, gu = tid % GT, k1 = 8 * grp + gu % 8, r = gu / 8, k2 = (r & 1) * HN + (r >> 1);
+  C* const w1p = sW + k1 * PS + G::off(k2);
+  C* const w2p = sW + k1 * PS + r;
+  const int x2 = r, x3 = k1, wid = tid / 32;
+  C* const w3p = sW + G::off(x2) + x3;
+
+  // second pass, in place
+  auto pass2 = [&](auto sgn) {
+    constexpr int S = decltype(sgn)::value;
+    C x[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = w2p[G::off(j)];
+    cfft<N, S>(x);
+#pragma unroll
+    for (int j = 0; j < N; ++j) w2p[G::off(j)] = x[j];
   };
-  auto phase_store = [&](C e, int slot) {
-    if (tid < 3 * N) {
-      C* dst = sPh + slot * PHS;
-      dst[tid] = e;
-      if (tid % N == NY) {
-        const C ce = mk<C>(e.x, -e.y);
-        dst[3 * N + tid / N] = cmul(ce, ce);
+  // axis phases e^{i fac_p s_q[ax] l0[k]} of (p, q) and Theta_ax =
+  // e^{i fac_p N s_q[ax]} = conj(e^{i fac_p s_q[ax] l0[N/2]})^2.  Nyquist
+  // threads carry one or two entries each.
+  constexpr int NPH = (3 * N + G::NQ - 1) / G::NQ;
+  auto phase_fetch = [&](int pq, CM (&e)[NPH]) {
+#pragma unroll
+    for (int i = 0; i < NPH; ++i) {
+      const int n = tq + i * G::NQ;
+      e[i] = n < 3 * N ? a.phase[(size_t)pq * 3 * N + n] : mk<CM>(T(0), T(0));
+    }
+  };
+  auto phase_store = [&](const CM (&e)[NPH], int slot) {
+#pragma unroll
+    for (int i = 0; i < NPH; ++i) {
+      const int n = tq + i * G::NQ;
+      CM* dst = sPh + slot * PHS;
+      if (n < 3 * N) dst[n] = e[i];
+      if (n < 3 * N && n % N == HN) {
+        const CM ce = mk<CM>(e[i].x, -e[i].y);
+        dst[3 * N + n / N] = cmul(ce, ce);
       }
     }
   };
-  // F at (k1, k2, k3) from the half spectrum
-  auto Fat = [&](int k1, int k2, int k3) -> C {
-    if (k3 <= NY) return sF[k1 * FS + k2 * H + k3];
-    const C c = sF[((N - k1) % N) * FS + ((N - k2) % N) * H + (N - k3)];
-    return mk<C>(c.x, -c.y);
-  };
-
   const int npts = a.pcount ? min(a.npts, *a.pcount) : a.npts;
   // work item = (point, chunk of radial nodes); with KP > 1 each chunk's
   // partial gain spectrum goes to its own scratch slice and the CTA that
@@ -150,325 +213,270 @@ __global__ void __launch_bounds__(CubeGeom<N>::NT, 1) vhs_cube_kernel(const VhsA
     const int gactive = waves > 0 ? (nitems + waves - 1) / waves : 0;
     if ((int)blockIdx.x >= gactive) return;  // uniform over the CTA, before any barrier
     if (tid == 0) {
+      mbar_init(&s_read, NM / 32);
+      s_gave_up = 0;
       s_kp = kp;
       s_ni = nitems;
       s_ga = gactive;
     }
   }
+  if (tid < 32) tmem_alloc(&s_tmem, G::TCOLS);
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  // this thread's lane and columns: F^ of line (k1, k2), then S of (x2, x3)
+  const uint32_t tmF = s_tmem + ((uint32_t)(tid / 32 % 4 * 32) << 16) + tid / 128 * G::TW, tmS = tmF + 2 * N * WD;
+  uint32_t rphase = 0;  // parity of s_read's current phase
+  constexpr int SC = N % 16 ? 8 : 16;  // values per step of the last pass
+  // F^ of this thread's line
+  auto load_line = [&](C (&x)[N]) {
+    uint32_t t[2 * N * WD];
+    tm_load(tmF, t);
+    tm_wait(t);
+#pragma unroll
+    for (int k = 0; k < N; ++k) x[k] = vmk(tm_get(t, 2 * k, T(0)), tm_get(t, 2 * k + 1, T(0)));
+  };
+
   for (int item = blockIdx.x; item < s_ni; item += s_ga) {
     const int ip = item / s_kp;
     const int pt = a.plist ? a.plist[a.pt0 + ip] : a.pt0 + ip;
     if ((unsigned)pt >= (unsigned)(a.nupts * a.neles)) continue;  // uniform over the CTA
-    const int upt = pt / a.neles, elem = pt % a.neles;
     if (tid == 0) {
       const int ch = item % s_kp;
       s_it[0] = ch * a.P / s_kp;
       s_it[1] = (ch + 1) * a.P / s_kp;
-      s_it[2] = upt;
-      s_it[3] = elem;
+      s_it[2] = pt / a.neles;
+      s_it[3] = pt % a.neles;
     }
 
-    // ---- F = FFT(f) / V, kept for k3 <= N/2 ---------------------------------
+    // ---- F^ = (1 + i) FFT(f) / V ---------------------------------------------
     if (is_main) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM;  // line (x1, x2) along x3
-        C x[N];
+      const int64_t b0 = soa_ix(pt / a.neles, a.ldim, pt % a.neles, (int64_t)(k1 * N + k2) * N, V, a.soasz);
+      C x[N];
 #pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = mk<C>(a.f[soa_ix(upt, a.ldim, elem, (int64_t)L * N + k, V, a.soasz)], 0.f);
-        fft<float, N, -1>(x);
+      for (int k = 0; k < N; ++k) x[k] = vmk(a.f[b0 + (int64_t)k * a.soasz], T(0));
+      cfft<N, -1>(x);
 #pragma unroll
-        for (int k = 0; k < N; ++k) sW[L * LP + k] = x[k];
-      }
+      for (int k = 0; k < N; ++k) w1p[k] = x[k];
+    }
+    __syncthreads();
+    if (is_main) pass2(std::integral_constant<int, -1>{});
+    __syncthreads();
+    if (is_main) {
+      const T iv = T(1) / T(V);
+      C x[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
+      cfft<N, -1>(x);
+#pragma unroll
+      for (int i = 0; i < N; ++i) w3p[i * PS] = vmul(mul_1i<1>(x[i]), vmk(iv, iv));
     }
     __syncthreads();
     if (is_main) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM, x1 = L / N, k3 = L % N;  // line (x1, k3) along x2
-        C x[N];
+      uint32_t t[2 * N * WD];
 #pragma unroll
-        for (int j = 0; j < N; ++j) x[j] = sW[(x1 * N + j) * LP + k3];
-        fft<float, N, -1>(x);
-#pragma unroll
-        for (int j = 0; j < N; ++j) sW[(x1 * N + j) * LP + k3] = x[j];
+      for (int i = 0; i < N; ++i) {
+        const C v = w1p[i];
+        tm_put(t, 2 * i, cre(v));
+        tm_put(t, 2 * i + 1, cim(v));
       }
-    }
-    __syncthreads();
-    if (is_main) {
+      tm_store(tmF, t);
+      tmem_store_wait();
+    } else {
 #pragma unroll 1
-      for (int L = tid; L < N * H; L += NM) {
-        const int k2 = L / H, k3 = L % H;  // line (k2, k3) along x1, k3 <= N/2
-        C x[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = sW[(i * N + k2) * LP + k3];
-        fft<float, N, -1>(x);
-#pragma unroll
-        for (int i = 0; i < N; ++i) sF[i * FS + k2 * H + k3] = cscale(x[i], invV);
+      for (int t = tq; t < 3 * N * N; t += G::NQ) {
+        const int k = t / (3 * N), line = t % (3 * N), which = line / N, j = line % N;
+        sN[t] = which == 0   ? sW[HN * PS + G::off(j) + k]
+                : which == 1 ? sW[j * PS + G::off(HN) + k]
+                             : sW[j * PS + G::off(k) + HN];
       }
+      CM e[NPH];
+      phase_fetch(s_it[0] * a.M, e);
+      phase_store(e, 0);
     }
-    phase_store(phase_fetch(s_it[0] * a.M), 0);
     __syncthreads();
 
     // ---- gain: fC = sum_p w1_p FFT(sum_q Re S_pq) ---------------------------
-    int slot = 0;
+    // Both kinds of threads run the same sequence of CTA-wide barriers: one
+    // per (p, q) and two per p.
+    if (is_main) {
+      int slot = 0;
 #pragma unroll 1
-    for (int p = s_it[0]; p < s_it[1]; ++p) {
-      float S0[N], S1[N];
-#pragma unroll
-      for (int k = 0; k < N; ++k) S0[k] = S1[k] = 0.f;
+      for (int p = s_it[0]; p < s_it[1]; ++p) {
 #pragma unroll 1
-      for (int q = 0; q < a.M; ++q) {
-        const int pq = p * a.M + q;
-        const C* ph = sPh + slot * PHS;
-        const C th1 = ph[3 * N], th2 = ph[3 * N + 1], th3 = ph[3 * N + 2];
-        const C phn = pq + 1 < npq ? phase_fetch(pq + 1) : mk<C>(0.f, 0.f);
-        // pass 1: R lines (k1, k2) along k3 | Nyquist first axes.
-        // m = Re((E + E t)(1 - i)) / 2 with E = E1 E2 E3[k3] and t the
-        // Nyquist factor (1 off the planes): per line A = (E12 + E12 t12)
-        // (1 - i) / 2 (A3 on the k3 = N/2 plane), then m = Re(A E3[k3]).
-        if (is_main && !IL1) {
-#pragma unroll 1
-          for (int r = 0; r < 2; ++r) {
-            const int L = tid + r * NM, k1 = L / N, k2 = L % N;
-            const C E12 = cmul(ph[k1], ph[N + k2]);
-            C t12 = mk<C>(1.f, 0.f);
-            if (k1 == NY) t12 = th1;
-            if (k2 == NY) t12 = cmul(t12, th2);
-            const C E12t = cmul(E12, t12);
-            const C s0 = cadd(E12, E12t), s3 = cadd(E12, cmul(E12t, th3));
-            const C A = mk<C>(0.5f * (s0.x + s0.y), 0.5f * (s0.y - s0.x));
-            const C A3 = mk<C>(0.5f * (s3.x + s3.y), 0.5f * (s3.y - s3.x));
+        for (int q = 0; q < a.M; ++q) {
+          // pass 1: m F^ along k3.  m = Re((E + E t)(1 - i)) / 2 with
+          // E = E12 E3[k3] and t the Nyquist factor (1 off the planes): per
+          // line A = (E12 + E12 t12) (1 - i) / 2 (A3 on the k3 = N/2 plane),
+          // then m = Re(A E3[k3])
+          {
+            const CM* ph = sPh + slot * PHS;
+            const CM E12 = cmul(ph[k1], ph[N + k2]);
+            CM Et = E12;
+            if (k1 == HN) Et = cmul(Et, ph[3 * N]);
+            if (k2 == HN) Et = cmul(Et, ph[3 * N + 1]);
+            const CM s0 = cadd(E12, Et), s3 = cadd(E12, cmul(Et, ph[3 * N + 2]));
+            const CM A = mk<CM>(T(0.5) * (s0.x + s0.y), T(0.5) * (s0.y - s0.x));
+            const CM A3 = mk<CM>(T(0.5) * (s3.x + s3.y), T(0.5) * (s3.y - s3.x));
             C x[N];
+            load_line(x);
+            // e3[N - k] = conj e3[k]
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-              const C e3 = ph[2 * N + k];
-              const C& Ak = k == NY ? A3 : A;
-              x[k] = cscale(Fat(k1, k2, k), Ak.x * e3.x - Ak.y * e3.y);
+            for (int k = 0; k <= HN; ++k) {
+              const CM e = ph[2 * N + k];
+              const CM& Ak = k == HN ? A3 : A;
+              const T c = Ak.x * e.x, m = c - Ak.y * e.y;
+              x[k] = vmk(cre(x[k]) * m, cim(x[k]) * m);
+              if (k > 0 && k < HN) {
+                const T n = c + Ak.y * e.y;
+                x[N - k] = vmk(cre(x[N - k]) * n, cim(x[N - k]) * n);
+              }
             }
-            fft<float, N, +1>(x);
+            cfft<N, 1>(x);
+            mbar_wait_bounded(&s_read, rphase ^ 1, a.err, &s_gave_up);  // the previous cube is read
 #pragma unroll
-            for (int k = 0; k < N; ++k) sW[L * LP + k] = x[k];
+            for (int k = 0; k < N; ++k) w1p[k] = x[k];
           }
-        } else if (is_main) {  // IL1: both lines of the thread at once
-          auto coef = [&](int k1, int k2, C& A, C& A3) {
-            const C E12 = cmul(ph[k1], ph[N + k2]);
-            C t12 = mk<C>(1.f, 0.f);
-            if (k1 == NY) t12 = th1;
-            if (k2 == NY) t12 = cmul(t12, th2);
-            const C E12t = cmul(E12, t12);
-            const C s0 = cadd(E12, E12t), s3 = cadd(E12, cmul(E12t, th3));
-            A = mk<C>(0.5f * (s0.x + s0.y), 0.5f * (s0.y - s0.x));
-            A3 = mk<C>(0.5f * (s3.x + s3.y), 0.5f * (s3.y - s3.x));
-          };
-          const int L0 = tid, L1 = tid + NM;
-          const int a1 = L0 / N, a2 = L0 % N, b1 = L1 / N, b2 = L1 % N;
-          C Aa, Aa3, Ab, Ab3;
-          coef(a1, a2, Aa, Aa3);
-          coef(b1, b2, Ab, Ab3);
-          C x[N], y[N];
+          slot ^= 1;
+          bar_arrive(B_T, NT);        // done with the Nyquist tables of the previous (p, q)
+          bar_sync(B_G + grp, GT);    // this group's planes are complete
+          if constexpr (NM / 32 > 4) {
+            const unsigned t0 = clock();
+            while (clock() - t0 < (unsigned)(wid >> 2) * kStagger) {
+            }
+          }
+          pass2(std::integral_constant<int, 1>{});
+          bar_sync(B_ALL, NT);        // the cube and the Nyquist tables are complete
+          // pass 3: lines (x2, x3) along k1; S += Re P Im P + Re Nq Im Nq with
+          // Nq = s1 T1(x2, x3) + s2 T2(x1, x3) + s3 T3(x1, x2), s = (-1)^x
+          // (a common sign of Nq drops out: s3 Nq is formed)
+          C x[N];
+#pragma unroll
+          for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
+          __syncwarp();
+          if (tid % 32 == 0) mbar_arrive(&s_read);  // this warp's part of the cube may be overwritten
+          rphase ^= 1;
+          uint32_t t[N * WD];
+          tmem_store_wait();
+          tm_load(tmS, t);
+          cfft<N, 1>(x);
+          const T s3 = (x3 & 1) ? T(-1) : T(1), s23 = (x2 & 1) ? -s3 : s3;
+          const C t1 = vmul(sT1[x2 * N + x3], vmk(s3, s3)), ss = vmk(s23, s23);
+          tm_wait(t);
+#pragma unroll
+          for (int i = 0; i < N; ++i) {
+            const C u = sT3[x2 * (N + 1) + i];
+            const C n = vfma(sT2[i * N + x3], ss, (i & 1) ? vsub(u, t1) : vadd(u, t1));
+            const T s0 = q == 0 ? T(0) : tm_get(t, i, T(0));
+            tm_put(t, i, fma(cre(x[i]), cim(x[i]), fma(cre(n), cim(n), s0)));
+          }
+          tm_store(tmS, t);
+        }
+        // FFT(S_p): lines of the third pass along x1 from the accumulators,
+        // each thread to the entries it read last, then planes k1 <= N/2
+        {
+          C x[N];
+          tmem_store_wait();
+          uint32_t t[N * WD];
+          tm_load(tmS, t);
+          tm_wait(t);
+#pragma unroll
+          for (int i = 0; i < N; ++i) x[i] = vmk(tm_get(t, i, T(0)), T(0));
+          cfft<N, -1>(x);
+#pragma unroll
+          for (int i = 0; i <= HN; ++i) w3p[i * PS] = x[i];
+        }
+        bar_sync(B_ALL, NT);
+        if (k1 <= HN) pass2(std::integral_constant<int, -1>{});
+        bar_sync(B_ALL, NT);
+        if (k1 <= HN) {
+          // line (k1, k2) along x3.  All loads of the accumulated line are
+          // issued before its first store (the slices could alias w1 as far
+          // as the compiler knows)
+          const T* w1 = a.w1t + (size_t)p * V + k1 * N + k2;
+          CM* const fca = (s_kp == 1 ? fcg : a.fcp + (size_t)item * G::SL) + k1 * N + k2;
+          C x[N];
+#pragma unroll
+          for (int k = 0; k < N; ++k) x[k] = w1p[k];
+          cfft<N, -1>(x);
 #pragma unroll
           for (int k = 0; k < N; ++k) {
-            const C e3 = ph[2 * N + k];
-            const C& A0 = k == NY ? Aa3 : Aa;
-            const C& B0 = k == NY ? Ab3 : Ab;
-            x[k] = cscale(Fat(a1, a2, k), A0.x * e3.x - A0.y * e3.y);
-            y[k] = cscale(Fat(b1, b2, k), B0.x * e3.x - B0.y * e3.y);
+            const T w = __ldg(w1 + k * NN);
+            x[k] = vmul(x[k], vmk(w, w));
           }
-          fft<float, N, +1>(x);
-          fft<float, N, +1>(y);
+          if (p > s_it[0]) {
 #pragma unroll
-          for (int k = 0; k < N; ++k) {
-            sW[L0 * LP + k] = x[k];
-            sW[L1 * LP + k] = y[k];
+            for (int k = 0; k < N; ++k) x[k] = vadd(from_c(fca[k * G::NL]), x[k]);
           }
-        } else {
-          // n F on the Nyquist planes: plane 1 (k1 = N/2) lines over k3,
+#pragma unroll
+          for (int k = 0; k < N; ++k) fca[k * G::NL] = to_c(x[k]);
+        }
+      }
+    } else {
+      int slot = 0;
+#pragma unroll 1
+      for (int p = s_it[0]; p < s_it[1]; ++p) {
+#pragma unroll 1
+        for (int q = 0; q < a.M; ++q) {
+          const int pq = p * a.M + q;
+          CM phn[NPH];
+          if (pq + 1 < npq) phase_fetch(pq + 1, phn);
+          // n F^ on the Nyquist planes: plane 1 (k1 = N/2) lines over k3,
           // plane 2 (k2 = N/2, k1 != N/2) lines over k3, plane 3 (k3 = N/2,
           // k1, k2 != N/2) lines over k2.  On a line only the phase of the
-          // running axis changes, so n = Re(D (1 - i)) / 2 with
-          // D = E (1 - t) becomes n = Re(A e[k]) with one coefficient A per
-          // line (A3 where k meets the Nyquist index of the running axis),
-          // as for the main lines.  Addresses and conjugation are selects,
-          // so lines of different planes share a warp without divergence.
+          // running axis changes, so n = Re(D (1 - i)) / 2 with D = E (1 - t)
+          // becomes n = Re(A e[k]) with one coefficient A per line (A3 where
+          // k meets the Nyquist index of the running axis).
 #pragma unroll 1
           for (int line = tq; line < 3 * N; line += G::NQ) {
             const int which = line / N, j = line % N;
             const bool p3 = which == 2;
-            C Eb, tb;
-            if (which == 0) {
-              Eb = cmul(ph[NY], ph[N + j]);
-              tb = j == NY ? cmul(th1, th2) : th1;
-            } else if (which == 1) {
-              Eb = cmul(ph[j], ph[N + NY]);
-              tb = th2;
-            } else {
-              Eb = cmul(ph[j], ph[2 * N + NY]);
-              tb = th3;
-            }
-            C B = cmul(Eb, mk<C>(1.f - tb.x, -tb.y));
-            const C tb3 = cmul(tb, th3);
-            C B3 = p3 ? mk<C>(0.f, 0.f) : cmul(Eb, mk<C>(1.f - tb3.x, -tb3.y));
-            if (which != 0 && j == NY) B = B3 = mk<C>(0.f, 0.f);
-            const C A = mk<C>(0.5f * (B.x + B.y), 0.5f * (B.y - B.x));
-            const C A3 = mk<C>(0.5f * (B3.x + B3.y), 0.5f * (B3.y - B3.x));
-            const C* ev = ph + (p3 ? N : 2 * N);
-            // element k at lo + k sl (k <= N/2, or every k on plane 3), else
-            // conj(sF[hi - k]) (the mirrored point)
-            const int jm = (N - j) % N;
-            const int lo = which == 0 ? NY * FS + j * H : (which == 1 ? j * FS + NY * H : j * FS + NY);
-            const int sl = p3 ? H : 1;
-            const int hi = (which == 0 ? NY * FS + jm * H : jm * FS + NY * H) + N;
+            const CM* ph = sPh + slot * PHS;
+            const CM th1 = ph[3 * N], th2 = ph[3 * N + 1], th3 = ph[3 * N + 2];
+            const CM Eb = cmul(ph[which == 0 ? HN : j], ph[which == 0 ? N + j : p3 ? 2 * N + HN : N + HN]);
+            CM tb = which == 0 ? th1 : p3 ? th3 : th2;
+            if (which == 0 && j == HN) tb = cmul(tb, th2);
+            const CM tb3 = cmul(tb, th3);
+            CM B = cmul(Eb, mk<CM>(T(1) - tb.x, -tb.y));
+            CM B3 = p3 ? mk<CM>(T(0), T(0)) : cmul(Eb, mk<CM>(T(1) - tb3.x, -tb3.y));
+            if (which != 0 && j == HN) B = B3 = mk<CM>(T(0), T(0));
+            const CM A = mk<CM>(T(0.5) * (B.x + B.y), T(0.5) * (B.y - B.x));
+            const CM A3 = mk<CM>(T(0.5) * (B3.x + B3.y), T(0.5) * (B3.y - B3.x));
+            const CM* ev = ph + (p3 ? N : 2 * N);
             C x[N];
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-              C v;
-              if (k <= NY) {
-                v = sF[lo + k * sl];
-              } else {
-                const C c = sF[p3 ? lo + k * H : hi - k];
-                v = mk<C>(c.x, p3 ? c.y : -c.y);
-              }
-              const C& Ak = k == NY ? A3 : A;
-              const C e = ev[k];
-              x[k] = cscale(v, Ak.x * e.x - Ak.y * e.y);
+              const C v = sN[k * 3 * N + line];
+              const CM e = ev[k];
+              const CM& Ak = k == HN ? A3 : A;
+              const T n = Ak.x * e.x - Ak.y * e.y;
+              x[k] = vmk(cre(v) * n, cim(v) * n);
             }
-            fft<float, N, +1>(x);
-            C* T = which == 0 ? sT1 : (which == 1 ? sT2 : sT3);
+            cfft<N, 1>(x);
 #pragma unroll
-            for (int k = 0; k < N; ++k) T[j * LP + k] = x[k];
+            for (int k = 0; k < N; ++k) sX[line * (N + 1) + k] = x[k];
           }
-        }
-        if (pq + 1 < npq) phase_store(phn, slot ^ 1);
-        __syncthreads();
-        // pass 2: lines (k1, x3) along k2, both lines of a thread at once |
-        // Nyquist second axes (columns)
-        if (is_main) {
-          const int L0 = tid, L1 = tid + NM;
-          C* w0 = sW + (L0 / N) * N * LP + L0 % N;
-          C* w1 = sW + (L1 / N) * N * LP + L1 % N;
-          C x[N], y[N];
-#pragma unroll
-          for (int j = 0; j < N; ++j) {
-            x[j] = w0[j * LP];
-            y[j] = w1[j * LP];
-          }
-          fft<float, N, +1>(x);
-          fft<float, N, +1>(y);
-#pragma unroll
-          for (int j = 0; j < N; ++j) {
-            w0[j * LP] = x[j];
-            w1[j * LP] = y[j];
-          }
-        } else {
+          if (pq + 1 < npq) phase_store(phn, slot ^ 1);
+          slot ^= 1;
+          bar_sync(B_T, NT);  // every first axis is done, and no main thread reads the old tables
 #pragma unroll 1
           for (int line = tq; line < 3 * N; line += G::NQ) {
-            const int which = line / N, col = line % N;
-            C* T = which == 0 ? sT1 : (which == 1 ? sT2 : sT3);
+            const int which = line / N, j = line % N;
             C x[N];
 #pragma unroll
-            for (int j = 0; j < N; ++j) x[j] = T[j * LP + col];
-            fft<float, N, +1>(x);
+            for (int i = 0; i < N; ++i) x[i] = sX[(which * N + i) * (N + 1) + j];
+            cfft<N, 1>(x);
+            // element i of the column: T1[i][j], T2[i][j], T3[j][i]
+            C* const d = which == 0 ? sT1 + j : which == 1 ? sT2 + j : sT3 + j * (N + 1);
+            const int de = which == 2 ? 1 : N;
 #pragma unroll
-            for (int j = 0; j < N; ++j) T[j * LP + col] = x[j];
+            for (int i = 0; i < N; ++i) d[i * de] = x[i];
           }
+          bar_sync(B_ALL, NT);
         }
-        __syncthreads();
-        // pass 3: lines (x2, x3) along k1, both lines at once;
-        // S += Re R^2 + Re Nq^2
-        if (is_main) {
-          const int L0 = tid, L1 = tid + NM;
-          const int a2 = L0 / N, a3 = L0 % N, b2 = L1 / N, b3 = L1 % N;
-          C x[N], y[N];
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            x[i] = sW[(i * N + a2) * LP + a3];
-            y[i] = sW[(i * N + b2) * LP + b3];
-          }
-          fft<float, N, +1>(x);
-          fft<float, N, +1>(y);
-          const C ta = sT1[a2 * LP + a3], tb = sT1[b2 * LP + b3];
-          const float sa2 = (a2 & 1) ? -1.f : 1.f, sa3 = (a3 & 1) ? -1.f : 1.f;
-          const float sb2 = (b2 & 1) ? -1.f : 1.f, sb3 = (b3 & 1) ? -1.f : 1.f;
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            const float s1 = (i & 1) ? -1.f : 1.f;
-            {
-              const C t2 = sT2[i * LP + a3], t3 = sT3[i * LP + a2];
-              const float nr = s1 * ta.x + sa2 * t2.x + sa3 * t3.x;
-              const float ni = s1 * ta.y + sa2 * t2.y + sa3 * t3.y;
-              S0[i] += x[i].x * x[i].x - x[i].y * x[i].y + nr * nr - ni * ni;
-            }
-            {
-              const C t2 = sT2[i * LP + b3], t3 = sT3[i * LP + b2];
-              const float nr = s1 * tb.x + sb2 * t2.x + sb3 * t3.x;
-              const float ni = s1 * tb.y + sb2 * t2.y + sb3 * t3.y;
-              S1[i] += y[i].x * y[i].x - y[i].y * y[i].y + nr * nr - ni * ni;
-            }
-          }
-        }
-        slot ^= 1;
-        __syncthreads();
+        bar_sync(B_ALL, NT);
+        bar_sync(B_ALL, NT);
       }
-
-      // FFT(S_p): lines (x2, x3) along x1 straight from the accumulators
-      if (is_main) {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int L = tid + r * NM, x2 = L / N, x3 = L % N;
-          C x[N];
-#pragma unroll
-          for (int i = 0; i < N; ++i) x[i] = mk<C>(r == 0 ? S0[i] : S1[i], 0.f);
-          fft<float, N, -1>(x);
-#pragma unroll
-          for (int i = 0; i < N; ++i) sW[(i * N + x2) * LP + x3] = x[i];
-        }
-      }
-      __syncthreads();
-      if (is_main) {
-#pragma unroll 1
-        for (int r = 0; r < 2; ++r) {
-          const int L = tid + r * NM, k1 = L / N, x3 = L % N;
-          C x[N];
-#pragma unroll
-          for (int j = 0; j < N; ++j) x[j] = sW[(k1 * N + j) * LP + x3];
-          fft<float, N, -1>(x);
-#pragma unroll
-          for (int j = 0; j < N; ++j) sW[(k1 * N + j) * LP + x3] = x[j];
-        }
-      }
-      __syncthreads();
-      if (is_main) {
-        const float* w1 = a.w1t + (size_t)p * V;
-#pragma unroll 1
-        for (int r = 0; r < 2; ++r) {
-          const int L = tid + r * NM;  // line (k1, k2) along k3
-          // fC and w1 with the last axis outermost ([k3][L]): a warp's
-          // accesses are 32 consecutive entries.  All loads of the line are
-          // issued before its first store (fC and w1 could alias as far as
-          // the compiler knows, which would otherwise order each load after
-          // the previous store): one round trip per line, not one per entry.
-          C x[N];
-#pragma unroll
-          for (int k = 0; k < N; ++k) x[k] = sW[L * LP + k];
-          fft<float, N, -1>(x);
-#pragma unroll
-          for (int k = 0; k < N; ++k) x[k] = cscale(x[k], w1[k * NN + L]);
-          C* const fca = s_kp == 1 ? fcg : a.fcp + (size_t)item * V;
-          if (p > s_it[0]) {
-            C acc[N];
-#pragma unroll
-            for (int k = 0; k < N; ++k) acc[k] = fca[k * NN + L];
-#pragma unroll
-            for (int k = 0; k < N; ++k) fca[k * NN + L] = cadd(acc[k], x[k]);
-          } else {
-#pragma unroll
-            for (int k = 0; k < N; ++k) fca[k * NN + L] = x[k];
-          }
-        }
-      }
-      __syncthreads();
     }
 
     if (s_kp > 1) {
@@ -481,124 +489,117 @@ __global__ void __launch_bounds__(CubeGeom<N>::NT, 1) vhs_cube_kernel(const VhsA
       __threadfence();
     }
 
-    // ---- Q = prefac (Re IFFT(fC) - f IFFT(b2 F)) ----------------------------
-    // Two transforms: fC, summed from FP32 transforms of real fields, is
-    // conjugate-even only to round-off, and packing it with b2 F into one
-    // transform would leak that round-off into the loss term as a constant
-    // times f (a momentum error proportional to rho u).
-    auto pass23 = [&]() {  // the pass along k2, in place, between barriers
-      __syncthreads();
-      if (is_main) {
-#pragma unroll 1
-        for (int r = 0; r < 2; ++r) {
-          const int L = tid + r * NM;
-          C* w = sW + (L / N) * N * LP + L % N;
-          C x[N];
-#pragma unroll
-          for (int j = 0; j < N; ++j) x[j] = w[j * LP];
-          fft<float, N, +1>(x);
-#pragma unroll
-          for (int j = 0; j < N; ++j) w[j * LP] = x[j];
-        }
-      }
-      __syncthreads();
-    };
-    // Lf = IFFT(b2 F): b2 F is built conjugate-even from the half spectrum.
-    // F is not needed after this transform's first pass, so its storage
-    // takes the real Lf values (slot v of each thread's own lines).
-    float* const sLf = reinterpret_cast<float*>(sF);
-    static_assert(2 * N * FS >= V, "Lf fits in the spectrum storage");
+    // ---- Q = prefac (Re IFFT(fC) - f Re IFFT(b2 F)) ----------------------------
+    // Two transforms: fC, summed from FP32 transforms, carries round-off, and
+    // packing it with b2 F into one transform would leak that round-off into
+    // the loss term as a constant times f (a momentum error proportional to
+    // rho u).  The transform of b2 F^ gives (1 + i) times the real collision
+    // frequency: its real part, kept where S was.
     if (is_main) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM, k1 = L / N, k2 = L % N;
-        C x[N];
+      const T* b2 = a.b2t + k1 * N + k2;
+      C x[N];
+      load_line(x);
 #pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = cscale(Fat(k1, k2, k), a.b2t[k * NN + L]);
-        fft<float, N, +1>(x);
-#pragma unroll
-        for (int k = 0; k < N; ++k) sW[L * LP + k] = x[k];
+      for (int k = 0; k < N; ++k) {
+        const T b = __ldg(b2 + k * NN);
+        x[k] = vmul(x[k], vmk(b, b));
       }
-    }
-    pass23();
-    if (is_main) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM, x2 = L / N, x3 = L % N;
-        C x[N];
+      cfft<N, 1>(x);
 #pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = sW[(i * N + x2) * LP + x3];
-        fft<float, N, +1>(x);
-#pragma unroll
-        for (int i = 0; i < N; ++i) sLf[(i * N + x2) * N + x3] = x[i].x;
-      }
+      for (int k = 0; k < N; ++k) w1p[k] = x[k];
     }
     __syncthreads();
-    // QG = Re IFFT(fC)
+    if (is_main) pass2(std::integral_constant<int, 1>{});
+    __syncthreads();
     if (is_main) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM;
-        C x[N];
-        if (s_kp == 1) {
+      C x[N];
 #pragma unroll
-          for (int k = 0; k < N; ++k) x[k] = fcg[k * NN + L];
-        } else {
-          // the chunks' slices, summed in a fixed order (L2 reads: other
-          // CTAs wrote them)
+      for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
+      cfft<N, 1>(x);
+      uint32_t t[N * WD];
 #pragma unroll
-          for (int k = 0; k < N; ++k) x[k] = mk<C>(0.f, 0.f);
-#pragma unroll 1
-          const int kp = s_kp, i0 = item - item % kp;
-          for (int c = 0; c < kp; ++c) {
-            const C* src = a.fcp + (size_t)(i0 + c) * V + L;
-#pragma unroll
-            for (int k = 0; k < N; ++k) x[k] = cadd(x[k], __ldcg(src + k * NN));
-          }
-        }
-        fft<float, N, +1>(x);
-#pragma unroll
-        for (int k = 0; k < N; ++k) sW[L * LP + k] = x[k];
-      }
+      for (int i = 0; i < N; ++i) tm_put(t, i, cre(x[i]));
+      tm_store(tmS, t);
+      tmem_store_wait();
     }
-    pass23();
-    double mom[5] = {0, 0, 0, 0, 0};
+    __syncthreads();
+    // QG = Re IFFT(fC); the chunks' slices are summed in a fixed order (L2
+    // reads: other CTAs wrote them).  Planes k1 > N/2 are the conjugate
+    // mirror of k1 < N/2.
     if (is_main) {
+      const bool mir = k1 > HN;
+      const int line = mir ? (N - k1) * N + (N - k2) % N : k1 * N + k2;
+      const int kp = s_kp, i0 = item - item % kp;
+      const CM* src = (kp == 1 ? fcg : a.fcp + (size_t)i0 * G::SL) + line;
+      C x[N];
+#pragma unroll
+      for (int k = 0; k < N; ++k) x[k] = from_c(__ldcg(src + k * G::NL));
 #pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM, x2 = L / N, x3 = L % N;
-        // bank entry of v = i N^2 + L is b0 + i st (v enters the AoSoA
-        // index linearly); f of this line is loaded first, every load
-        // issued before the first store of Q (which may alias f as far as
-        // the compiler knows)
-        const int64_t b0 = soa_ix(s_it[2], a.ldim, s_it[3], L, V, a.soasz), st = (int64_t)NN * a.soasz;
-        C x[N];
+      for (int c = 1; c < kp; ++c) {
+        src += G::SL;
 #pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = sW[(i * N + x2) * LP + x3];
-        fft<float, N, +1>(x);
-        float fl[N];
+        for (int k = 0; k < N; ++k) x[k] = vadd(x[k], from_c(__ldcg(src + k * G::NL)));
+      }
+      if (mir) {
+        // x[k] <- conj x[-k]
+        sfor<1, HN>([&](auto kc) {
+          constexpr int k = decltype(kc)::value;
+          const C t = x[k];
+          x[k] = vmk(cre(x[N - k]), -cim(x[N - k]));
+          x[N - k] = vmk(cre(t), -cim(t));
+        });
+        x[0] = vmk(cre(x[0]), -cim(x[0]));
+        x[HN] = vmk(cre(x[HN]), -cim(x[HN]));
+      }
+      cfft<N, 1>(x);
 #pragma unroll
-        for (int i = 0; i < N; ++i) fl[i] = a.f[b0 + i * st];
+      for (int k = 0; k < N; ++k) w1p[k] = x[k];
+    }
+    __syncthreads();
+    if (is_main) pass2(std::integral_constant<int, 1>{});
+    __syncthreads();
+    double mom[5] = {0, 0, 0, 0, 0};
+    // bank entry of v = i N^2 + x2 N + x3 is b0 + i st: v enters the AoSoA index
+    // linearly
+    const int64_t b0 = soa_ix(s_it[2], a.ldim, s_it[3], x2 * N + x3, V, a.soasz), st = (int64_t)NN * a.soasz;
+    if (is_main) {
+      C x[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-          const int64_t v = (int64_t)(i * N + x2) * N + x3;
-          const float qq = a.prefac * (x[i].x - fl[i] * sLf[v]);
-          if (!a.project) {
-            a.Q[b0 + i * st] = qq;
-            continue;
-          }
-          sW[(i * N + x2) * LP + x3].x = qq;  // this thread's own slot
-          {
+      for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
+      cfft<N, 1>(x);
+      sfor<0, N / SC>([&](auto cc) {
+        constexpr int c = decltype(cc)::value;
+        uint32_t t[SC * WD];
+        tm_load(tmS + SC * c * WD, t);
+        // f first, every load of the step issued before its first store of Q
+        // (which may alias f as far as the compiler knows)
+        T fl[SC];
+#pragma unroll
+        for (int h = 0; h < SC; ++h) fl[h] = a.f[b0 + (SC * c + h) * st];
+        tm_wait(t);
+#pragma unroll
+        for (int h = 0; h < SC; ++h) {
+          const int i = SC * c + h;
+          const T qq = a.prefac * (cre(x[i]) - fl[h] * tm_get(t, h, T(0)));
+          if (!a.project) a.Q[b0 + i * st] = qq;
+          tm_put(t, h, qq);
+        }
+        if (a.project) {
+#pragma unroll
+          for (int h = 0; h < SC; ++h) {
+            const int v = (SC * c + h) * NN + x2 * N + x3;
             const double c0 = a.cvec[v], c1 = a.cvec[V + v], c2 = a.cvec[2 * V + v];
-            const double d = (double)qq;
+            const double d = (double)tm_get(t, h, T(0));
             mom[0] += d;
             mom[1] += d * c0;
             mom[2] += d * c1;
             mom[3] += d * c2;
             mom[4] += d * (c0 * c0 + c1 * c1 + c2 * c2);
           }
+          tm_store(tmS + SC * c * WD, t);
         }
-      }
+      });
+      tmem_store_wait();
     }
     if (a.project) {  // uniform: every thread takes part in the reduction
 #pragma unroll
@@ -620,25 +621,28 @@ __global__ void __launch_bounds__(CubeGeom<N>::NT, 1) vhs_cube_kernel(const VhsA
         sLam[tid] = l;
       }
       __syncthreads();
-    }
-    if (is_main && a.project) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        const int L = tid + r * NM, x2 = L / N, x3 = L % N;
+      if (is_main) {
+        sfor<0, N / SC>([&](auto cc) {
+          constexpr int c = decltype(cc)::value;
+          uint32_t t[SC * WD];
+          tm_load(tmS + SC * c * WD, t);
+          tm_wait(t);
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-          const int64_t v = (int64_t)(i * N + x2) * N + x3;
-          const double c0 = a.cvec[v], c1 = a.cvec[V + v], c2 = a.cvec[2 * V + v];
-          const float qq = (float)((double)sW[(i * N + x2) * LP + x3].x -
-                                   (sLam[0] + sLam[1] * c0 + sLam[2] * c1 + sLam[3] * c2 +
-                                    sLam[4] * (c0 * c0 + c1 * c1 + c2 * c2)));
-          a.Q[soa_ix(s_it[2], a.ldim, s_it[3], v, V, a.soasz)] = qq;
-        }
+          for (int h = 0; h < SC; ++h) {
+            const int v = (SC * c + h) * NN + x2 * N + x3;
+            const double c0 = a.cvec[v], c1 = a.cvec[V + v], c2 = a.cvec[2 * V + v];
+            a.Q[b0 + (SC * c + h) * st] =
+                (T)((double)tm_get(t, h, T(0)) - (sLam[0] + sLam[1] * c0 + sLam[2] * c1 + sLam[3] * c2 +
+                                                         sLam[4] * (c0 * c0 + c1 * c1 + c2 * c2)));
+          }
+        });
       }
     }
     if (s_kp > 1 && tid == 0) a.pdone[item / s_kp] = 0;  // every chunk has counted: ready for the next launch
     __syncthreads();  // the work cube and fC are reused by the next point
   }
+  __syncthreads();
+  if (tid < 32) tmem_dealloc(s_tmem, G::TCOLS);
 }
 
 }  // namespace dgfs

@@ -54,7 +54,10 @@ def tune_vhs(sm, fin, fout, npts=None, reps=2, cache=True, verbose=False):
            f'{npts}|{sm._project}')
     db = _load() if cache else {}
     variants = sm.variants()
-    if key in db and db[key]['index'] < len(variants):
+    # an entry counts only while its index still names the shape it was
+    # measured on (the list of compiled shapes changes with the library)
+    if key in db and db[key]['index'] < len(variants) and \
+            db[key].get('variant') == variants[db[key]['index']]:
         sm.select(db[key]['index'])
         return db[key]
 
