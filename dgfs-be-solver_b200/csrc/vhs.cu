@@ -13,7 +13,6 @@
 #include "../../include/dgfs_b200.h"
 #include "dgfs_internal.h"
 #include "vhs_push.cuh"
-#include "vhs_pair.cuh"
 #include "vhs_variant.h"
 
 namespace dgfs {
@@ -116,64 +115,26 @@ template <typename T, int N, int C, int MINB> static VhsVariant make_push() {
   return v;
 }
 
-template <typename T, int N, int LPT>
-static cudaError_t launch_pair(const VhsArgs<T>& a, int nclusters, cudaStream_t s) {
-  using G = PairGeom<T, N, LPT>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nclusters * 2, 1, 1);
-  cfg.blockDim = dim3(G::NT, 1, 1);
-  cfg.dynamicSmemBytes = G::SMEM_CX * sizeof(cx<T>);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, vhs_pair_kernel<T, N, LPT>, a);
-}
-
-// two-CTA kernel (FP32 N = 32, FP64 N = 24; kind 3 in dgfs_vhs_variant_kind);
-// LPT lines per main thread and pass (db reports LPT - 1)
-template <typename T, int N, int LPT> static VhsVariant make_pair() {
-  using G = PairGeom<T, N, LPT>;
-  VhsVariant v{};
-  v.prec = sizeof(T) == 8 ? 64 : 32;
-  v.N = N;
-  v.C = 2;
-  v.db = LPT - 1;
-  v.push = 3;
-  v.minb = 1;
-  v.threads = G::NT;
-  v.smem = G::SMEM_CX * sizeof(cx<T>);
-  v.scratch_cx = G::SCRATCH;
-  v.fn = (const void*)vhs_pair_kernel<T, N, LPT>;
-  if constexpr (sizeof(T) == 8) v.launch64 = launch_pair<T, N, LPT>;
-  else v.launch32 = launch_pair<T, N, LPT>;
-  return v;
-}
-
 // Compiled launch shapes: (precision, N, cluster size, double-buffered
 // exchange, minimum CTAs per SM for the register budget).  The first entry
 // of each (precision, N) family is the default: the single-CTA kernel where a
 // point fits one SM (FP32 N = 24: 4.2 ms against 20 ms for the best cluster
 // shape on 576 points; FP32 N = 16: 0.49 ms against 1.16 ms on 592 points;
 // FP64 N = 16: 71 us against 204 us on one point), else the two-CTA kernel
-// (FP64 N = 24: 15 ms against 50 ms on 576 points; FP32 N = 32: 552 ms against
+// (FP64 N = 24: 11 ms against 50 ms on 576 points; FP32 N = 32: 450 ms against
 // 1,695 ms on 10,368); the autotuner times the rest.
 static const std::vector<VhsVariant>& variants() {
   static const std::vector<VhsVariant> v = {
       make_push<double, 8, 1, 4>(),             cube_variant(64, 16),
       make_push<double, 16, 4, 2>(),            make_push<double, 16, 2, 1>(),
-      make_pair<double, 24, 1>(),               make_pair<double, 24, 2>(),
+      pair_variant(64, true),                   pair_variant(64, false),
       make_push<double, 24, 8, 1>(),            make_push<double, 24, 12, 1>(),
       make_push<double, 32, 16, 1>(),           make_push<float, 8, 1, 4>(),
       cube_variant(32, 16),                     make_push<float, 16, 2, 2>(),
       make_push<float, 16, 4, 4>(),             cube_variant(32, 24),
       make_push<float, 24, 8, 2>(),             make_push<float, 24, 4, 1>(),
-      make_push<float, 24, 12, 3>(),            make_pair<float, 32, 2>(),
-      make_pair<float, 32, 1>(),                make_push<float, 32, 16, 2>(),
+      make_push<float, 24, 12, 3>(),            pair_variant(32, true),
+      pair_variant(32, false),                  make_push<float, 32, 16, 2>(),
       make_push<float, 32, 8, 1>(),             cube_variant(32, 8),
       make_variant<double, 8, 1, true, 4>(),    make_variant<double, 8, 2, true, 8>(),
       make_variant<double, 16, 4, true, 2>(),   make_variant<double, 16, 2, true, 1>(),

@@ -28,5 +28,8 @@ constexpr int kCubeSlices = 24;
 // single-CTA kernel (kind 2 in dgfs_vhs_variant_kind): FP32 N = 8, 16, 24 and
 // FP64 N = 16
 VhsVariant cube_variant(int prec, int N);
+// two-CTA kernel (kind 3): FP32 N = 32 and FP64 N = 24; own: Nyquist lines on
+// threads of their own
+VhsVariant pair_variant(int prec, bool own);
 
 }  // namespace dgfs
