@@ -12,7 +12,12 @@
 
 using namespace dgfs;
 
+constexpr int kFacMax = 4;  // points per direction of the factored operators
+
 struct dgfs_dg {
+  // 1D factors of m0, m132, m3 (DgFac); fac: they reproduce the matrices
+  bool fac;
+  double fl[2][kFacMax], fd[kFacMax][kFacMax], fla[kFacMax][kFacMax], flc[2][kFacMax];
   int prec, D, U, F, V, E, nb, ngroups, device, nhalo, nsend;
   int shape;  // residual launch shape (kDgShapes)
   long long ldim_u, ldim_f;
@@ -41,6 +46,25 @@ struct DgShape {
 };
 constexpr DgShape kDgShapes[] = {{8, 0, 0}, {8, 1, 0}, {8, 1, 2}, {16, 1, 2}, {4, 0, 0}, {4, 1, 0}, {2, 1, 0}};
 constexpr int kDgNumShapes = sizeof(kDgShapes) / sizeof(kDgShapes[0]);
+// The shape a handle starts with: Runge-Kutta terms loaded ahead (every
+// measured mesh gains 10-25 %) and as many velocities per warp as leave enough
+// CTAs.  w = waves of 8-velocity CTAs; measured stage times in us with 8 / 4 / 2
+// velocities per warp: FP32 p = 2, 10 elements, N = 16 (w = 0.1) 55 / 44 / 41;
+// FP32 p = 2, 64 elements, N = 24 (1.0) 82.8 / 82.0 / 83.7; FP32 p = 3, 40
+// elements, N = 24 (1.5) 160 / 142 / 141; FP64 p = 2, 91 elements, N = 24 (2.2)
+// 182 / 173 / 180; FP64 p = 3, 64 elements, N = 24 (2.9) 213 / 226 / 248; FP32
+// p = 2, 288 elements, N = 32 (10) 552 / 553 / 598; FP32 p = 3, 640 elements,
+// N = 32 (35) 2187 / 2285 / 2335.
+int default_shape(const dgfs_dg* h) {
+  const int per_sm = h->prec == 32 ? (h->U <= 9 ? 3 : 2) : (h->U <= 9 ? 2 : 1);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const double ctas = (double)((h->E + 31) / 32) * ((h->V + 63) / 64), w = ctas / ((double)sms * per_sm);
+  return w < 0.5 ? 6 : w < 2.5 ? 5 : 1;
+}
+static_assert(kDgShapes[1].vpt == 8 && kDgShapes[5].vpt == 4 && kDgShapes[6].vpt == 2 && kDgShapes[1].pf &&
+                  kDgShapes[5].pf && kDgShapes[6].pf,
+              "default_shape names these shapes");
 // Tensor-core residual shapes (FP32 only; dg_tc.cuh), numbered after the
 // SIMT shapes: velocities per warp of a 128-thread CTA, Runge-Kutta terms
 // always loaded ahead, CTAs per SM (0: 4 for p <= 2, 2 for p = 3, what the
@@ -182,6 +206,85 @@ template <typename T, int U, int F, int D> DgOps<T, U, F, D> make_ops(const dgfs
   return o;
 }
 
+template <typename T, int n> DgFac<T, n> make_fac(const dgfs_dg* h) {
+  DgFac<T, n> o;
+  for (int e = 0; e < 2; ++e)
+    for (int i = 0; i < n; ++i) {
+      o.l[e][i] = (T)h->fl[e][i];
+      o.lc[e][i] = (T)h->flc[e][i];
+    }
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) {
+      o.d[i][j] = (T)h->fd[i][j];
+      o.la[i][j] = (T)h->fla[i][j];
+    }
+  return o;
+}
+
+// 1D factors of the element operators (DgFac), and whether they reproduce
+// every entry of M0, M1 = M132 + M3 M2 (M2 = reference normal x M0) and M3 to
+// 1e-12 of the largest.  frfs's quadrilateral operators do to round-off; the
+// dense kernels take any other matrices.
+void dg_factor(dgfs_dg* h) {
+  h->fac = false;
+  const int U = h->U, F = h->F;
+  int n = 1;
+  while (n * n < U) ++n;
+  if (h->D != 2 || n * n != U || F != 4 * n || n < 2 || n > kFacMax) return;
+  const double *m0 = h->m0.data(), *m3 = h->m3.data();
+  static const double nref[4][2] = {{0, -1}, {1, 0}, {0, 1}, {-1, 0}};
+  std::vector<double> m1(h->m132);
+  for (int r = 0; r < U; ++r)
+    for (int f = 0; f < F; ++f)
+      for (int d = 0; d < 2; ++d)
+        for (int k = 0; k < U; ++k) m1[(size_t)r * 2 * U + d * U + k] += m3[r * F + f] * nref[f / n][d] * m0[f * U + k];
+  auto big = [](const double* m, size_t c) {
+    double b = 0;
+    for (size_t i = 0; i < c; ++i) b = std::fmax(b, std::fabs(m[i]));
+    return b;
+  };
+  const double t0 = 1e-12 * big(m0, (size_t)F * U), t1 = 1e-12 * big(m1.data(), m1.size()),
+               t3 = 1e-12 * big(m3, (size_t)U * F);
+  if (!(t0 > 0 && t1 > 0 && t3 > 0)) return;
+  int r0 = 0, q0 = 0;  // the largest entry of the bottom face's lift
+  for (int r = 0; r < U; ++r)
+    for (int t = 0; t < n; ++t)
+      if (std::fabs(m3[r * F + t]) > std::fabs(m3[r0 * F + q0])) r0 = r, q0 = t;
+  if (m3[r0 * F + q0] == 0) return;
+  const int i0 = r0 % n;
+  for (int i = 0; i < n; ++i) {
+    h->fl[0][i] = m0[i * n];
+    h->fl[1][i] = m0[(size_t)2 * n * U + i * n];
+    h->flc[0][i] = m3[(i * n + i0) * F + q0] / m3[r0 * F + q0];
+    h->flc[1][i] = m3[(i * n + i0) * F + 2 * n + q0] / m3[r0 * F + q0];
+    for (int k = 0; k < n; ++k) {
+      h->fd[i][k] = m1[(size_t)i * 2 * U + k];
+      h->fla[i][k] = m3[(r0 / n * n + i) * F + k];
+    }
+  }
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      const int r = j * n + i;
+      for (int t = 0; t < n; ++t) {
+        // faces bottom, right, top, left: trace of u at flux point t, lift
+        const double tr[4] = {i == t ? h->fl[0][j] : 0, j == t ? h->fl[1][i] : 0, i == t ? h->fl[1][j] : 0,
+                              j == t ? h->fl[0][i] : 0};
+        const double li[4] = {h->fla[i][t] * h->flc[0][j], h->fla[j][t] * h->flc[1][i], h->fla[i][t] * h->flc[1][j],
+                              h->fla[j][t] * h->flc[0][i]};
+        for (int f = 0; f < 4; ++f) {
+          if (!(std::fabs(m0[(size_t)(f * n + t) * U + r] - tr[f]) <= t0)) return;
+          if (!(std::fabs(m3[r * F + f * n + t] - li[f]) <= t3)) return;
+        }
+      }
+      for (int k = 0; k < U; ++k) {
+        const double dx = k / n == j ? h->fd[i][k % n] : 0, de = k % n == i ? h->fd[j][k / n] : 0;
+        if (!(std::fabs(m1[(size_t)r * 2 * U + k] - dx) <= t1)) return;
+        if (!(std::fabs(m1[(size_t)r * 2 * U + U + k] - de) <= t1)) return;
+      }
+    }
+  h->fac = true;
+}
+
 template <typename T, int U> DgMassOps<T, U> make_mass_ops(const dgfs_dg* h) {
   DgMassOps<T, U> o;
   for (int r = 0; r < U; ++r)
@@ -233,6 +336,13 @@ cudaError_t run_interp(const dgfs_dg* h, const void* u, int v0, int nv, cudaStre
   // shape (small meshes: more CTAs)
   const int vs = chunk_of(h->shape) / 8, vpt = vs <= 2 ? 2 : vs <= 4 ? 4 : kVpt;
   const dim3 grid((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * vpt - 1) / (8 * vpt)));
+  if (h->fac) {
+    constexpr int n = F / 4;
+    const DgFac<T, n> fac = make_fac<T, n>(h);
+    if (vpt <= 2) return launch_pdl(true, dg_interp_fac_kernel<T, n, 2>, grid, s, a, fac);
+    if (vpt <= 4) return launch_pdl(true, dg_interp_fac_kernel<T, n, 4>, grid, s, a, fac);
+    return launch_pdl(true, dg_interp_fac_kernel<T, n, kVpt>, grid, s, a, fac);
+  }
   const DgOps<T, U, F, D> ops = make_ops<T, U, F, D>(h);
   if (vpt <= 2) return launch_pdl(true, dg_interp_kernel<T, U, F, D, 2>, grid, s, a, ops);
   if (vpt <= 4) return launch_pdl(true, dg_interp_kernel<T, U, F, D, 4>, grid, s, a, ops);
@@ -247,11 +357,16 @@ constexpr int dg_default_mb() {
 template <typename T, int U, int F, int D, int VPT, int PF, int MB>
 cudaError_t launch_rhs(const dgfs_dg* h, const DgArgs<T>& a, int nv, cudaStream_t s) {
   constexpr int mb = MB ? MB : dg_default_mb<T, U, F, D>();
-  const dim3 grid((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * VPT - 1) / (8 * VPT)));
+  constexpr int n = F / 4;
+  dim3 grid((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * VPT - 1) / (8 * VPT)));
   // with halo rows the face values of other partitions arrive by a
   // collective on another stream: the residual then waits in plain stream
   // order for everything before it
-  return launch_pdl(h->nhalo == 0, dg_residual_kernel<T, U, F, D, VPT, PF, mb>, grid, s, a,
+  if (h->fac)
+    return launch_pdl(h->nhalo == 0, dg_residual_fac_kernel<T, n, VPT, PF, mb>, grid, s, a, make_fac<T, n>(h));
+  // matrices without 1D factors: one dense shape for every shape index
+  grid.y = (unsigned)((nv + 8 * kVpt - 1) / (8 * kVpt));
+  return launch_pdl(h->nhalo == 0, dg_residual_kernel<T, U, F, D, kVpt, 0, dg_default_mb<T, U, F, D>()>, grid, s, a,
                     make_ops<T, U, F, D>(h));
 }
 
@@ -418,11 +533,13 @@ extern "C" int dgfs_dg_create(const dgfs_dg_params* p, dgfs_dg** out) {
   h->m132.assign(p->m132, p->m132 + U * D * U);
   h->m3.assign(p->m3, p->m3 + U * F);
   if (p->m12) h->m12.assign(p->m12, p->m12 + U * U);
+  dg_factor(h);
   const size_t esz = h->prec == 64 ? 8 : 4;
   const long long row = nblk * 32 * (long long)h->V;
   const long long ldmod = 128 / (long long)esz;
   h->ldim_f = (row + ldmod - 1) / ldmod * ldmod;
   int rc = cudaGetDevice(&h->device) == cudaSuccess ? DGFS_OK : set_error(DGFS_ERR_CUDA, "no CUDA device");
+  h->shape = default_shape(h);
   if (!rc) rc = h->prec == 64 ? upload_geom<double>(h, p) : upload_geom<float>(h, p);
   if (!rc) rc = upload_int(&h->part, p->partner, (size_t)F * E);
   if (!rc) {
@@ -651,6 +768,13 @@ extern "C" int dgfs_dg_select(dgfs_dg* h, int idx) {
   if (idx < 0 || idx >= num_shapes(h))
     return set_error(DGFS_ERR_INVALID, "variant %d outside 0..%d", idx, num_shapes(h) - 1);
   h->shape = idx;
+  return DGFS_OK;
+}
+
+extern "C" int dgfs_dg_selected(const dgfs_dg* h, int* idx) {
+  clear_error();
+  if (!h || !idx) return set_error(DGFS_ERR_INVALID, "null argument");
+  *idx = h->shape;
   return DGFS_OK;
 }
 

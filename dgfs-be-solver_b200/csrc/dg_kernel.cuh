@@ -48,6 +48,21 @@ template <typename T, int U, int F, int D> struct DgOps {
   T m3[U][F];
 };
 
+// The same operators on a tensor-product element of n x n points (upt j n + i:
+// i along xi, j along eta; faces bottom, right, top, left with n flux points
+// each, in ascending order), as 1D factors:
+//   M0    traces l[0], l[1] at -1 and +1 along the axis across a face
+//   M1    the derivative d along either axis
+//   M3    lift = la (along the face) x lc[end] (across it)
+// dgfs_dg_create finds them in the matrices it is given and uses them only if
+// they reproduce every entry (dg_factor).
+template <typename T, int n> struct DgFac {
+  T l[2][n];
+  T d[n][n];
+  T la[n][n];
+  T lc[2][n];
+};
+
 template <typename T> struct DgArgs {
   int V, neles, v0, nv;
   int64_t ldim_u;          // leading dimension of solution banks
@@ -280,21 +295,20 @@ template <typename T, int N> __device__ __forceinline__ void lds16(const T* src,
 }
 
 // Ghost value of boundary point b at velocity v (bccflux.mako with the
-// bcs/*.mako kinds); nmv = |S^T n| n, whose sign tests equal the unit
-// normal's; ul the interior face value.
+// bcs/*.mako kinds) into *val, or true where it is the interior face value;
+// nmv = |S^T n| n, whose sign tests equal the unit normal's.
 template <typename T, int D>
-__device__ __forceinline__ T dg_ghost(const DgArgs<T>& a, int b, int v, int64_t e, int f, const T* c, const T* nmv,
-                                   T nc, T ul) {
+__device__ __forceinline__ bool dg_ghost(const DgArgs<T>& a, int b, int v, int64_t e, int f, const T* c, const T* nmv,
+                                         T* val) {
   const int kind = a.bkind[b], g = a.bgroup[b];
   if (kind == BC_WALL_DIFFUSE || kind == BC_INLET) {
     T fac = (c[0] - a.guw[g * 3]) * nmv[0];
 #pragma unroll
     for (int d = 1; d < D; ++d) fac = fma(c[d] - a.guw[g * 3 + d], nmv[d], fac);
-    if (fac < T(0)) {
-      const T fw = a.gfw[(int64_t)g * a.V + v];
-      return kind == BC_INLET ? fw : fw * (T)(-a.bcvals[2 * b] / a.bcvals[2 * b + 1]);
-    }
-    return ul;
+    if (!(fac < T(0))) return true;
+    const T fw = a.gfw[(int64_t)g * a.V + v];
+    *val = kind == BC_INLET ? fw : fw * (T)(-a.bcvals[2 * b] / a.bcvals[2 * b + 1]);
+    return false;
   }
   if (kind == BC_WALL_DIFFUSE_CYL) {
     // bcs/dgfs-wall-diffuse-cyl.mako: wall state of this boundary point
@@ -303,18 +317,23 @@ __device__ __forceinline__ T dg_ghost(const DgArgs<T>& a, int b, int v, int64_t 
     T fac = dc[0] * nmv[0];
 #pragma unroll
     for (int d = 1; d < D; ++d) fac = fma(dc[d], nmv[d], fac);
-    if (fac < T(0)) {
-      const T mx = exp(-(dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2]) / w[3]);
-      return mx * (T)(-a.bcvals[2 * b] / a.bcvals[2 * b + 1]);
-    }
-    return ul;
+    if (!(fac < T(0))) return true;
+    const T mx = exp(-(dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2]) / w[3]);
+    *val = mx * (T)(-a.bcvals[2 * b] / a.bcvals[2 * b + 1]);
+    return false;
   }
-  if (kind == BC_VANISH) return nc < T(0) ? T(0) : ul;
+  if (kind == BC_VANISH) {
+    T nc = nmv[0] * c[0];
+#pragma unroll
+    for (int d = 1; d < D; ++d) nc = fma(nmv[d], c[d], nc);
+    *val = T(0);
+    return !(nc < T(0));
+  }
   if (kind == BC_WALL_SPECULAR) {
-    const int vr = a.grefl[(int64_t)g * a.V + v];
-    return a.uf[aos32(f, a.ldim_f, e, vr, a.V)];
+    *val = a.uf[aos32(f, a.ldim_f, e, a.grefl[(int64_t)g * a.V + v], a.V)];
+    return false;
   }
-  return ul;  // outlet
+  return true;  // outlet
 }
 
 // Launch shapes (the autotuner's choice, dgfs_dg_select): VPT velocities per
@@ -404,7 +423,8 @@ __global__ void __launch_bounds__(256, MB)
         const int64_t pb = pl[f];
         if (pb < 0) {
           const int b = (int)(-pb - 1);
-          ur = b >= a.nb ? a.halo[(int64_t)(b - a.nb) * a.V + v] : dg_ghost<T, D>(a, b, v, e, f, c, nmv, nc, ul);
+          if (b >= a.nb) ur = a.halo[(int64_t)(b - a.nb) * a.V + v];
+          else if (dg_ghost<T, D>(a, b, v, e, f, c, nmv, &ur)) ur = ul;
         }
         // upwind flux (rusanov.mako:46-50) with the scaled normal
         const T fh = T(0.5) * nc * (ul + ur) + T(0.5) * fabs(nc) * (ul - ur);
@@ -432,6 +452,247 @@ __global__ void __launch_bounds__(256, MB)
 
     T rj[G::NR];
     lds16<T, G::NR / G::VW>(gl + G::OR, rj);
+    if constexpr (PF != 0) {
+      T* op_ = a.out + o;
+#pragma unroll
+      for (int r = 0; r < U; ++r, op_ += a.ldim_u) *op_ = fma(a.gamma, -rj[r] * R[r], K[r]);
+    } else {
+      const T* ap = a.A ? a.A + o : nullptr;
+      const T* bp = a.B ? a.B + o : nullptr;
+      const T* cp = a.Cq ? a.Cq + o : nullptr;
+      T* op_ = a.out + o;
+#pragma unroll
+      for (int r = 0; r < U; ++r) {
+        const T Rr = -rj[r] * R[r];
+        T res = a.gamma * (cp ? Rr + __ldg(cp) : Rr);
+        if (ap) res = fma(a.alpha, __ldg(ap), res);
+        if (bp) res = fma(a.beta, __ldg(bp), res);
+        *op_ = res;
+        op_ += a.ldim_u;
+        if (ap) ap += a.ldim_u;
+        if (bp) bp += a.ldim_u;
+        if (cp) cp += a.ldim_u;
+      }
+    }
+  }
+}
+
+// uf = M0 u from the 1D traces: n terms per flux point instead of n^2
+template <typename T, int n, int VPT>
+__global__ void __launch_bounds__(256) dg_interp_fac_kernel(const DgArgs<T> a, const DgFac<T, n> op) {
+  constexpr int U = n * n;
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t e = (int64_t)blockIdx.x * 32 + lane;
+  if (e >= a.neles) return;
+  const int vend = a.v0 + a.nv;
+  const int vbeg = a.v0 + (int)blockIdx.y * (8 * VPT) + w;
+#pragma unroll 1
+  for (int it = 0; it < VPT; ++it) {
+    const int v = vbeg + 8 * it;
+    if (v >= vend) break;
+    const int64_t o = ((int64_t)blockIdx.x * a.V + v) * 32 + lane;
+    T u[U];
+    const T* up = a.u + o;
+#pragma unroll
+    for (int i = 0; i < U; ++i, up += a.ldim_u) u[i] = __ldg(up);
+    T* fp = a.uf + o;
+#pragma unroll
+    for (int face = 0; face < 4; ++face) {
+      const int end = face == 1 || face == 2;
+      const bool xi = face & 1;  // the face is across the xi axis
+#pragma unroll
+      for (int t = 0; t < n; ++t, fp += a.ldim_f) {
+        T s = op.l[end][0] * u[xi ? t * n : t];
+#pragma unroll
+        for (int i = 1; i < n; ++i) s = fma(op.l[end][i], u[xi ? t * n + i : i * n + t], s);
+        *fp = s;
+      }
+    }
+  }
+}
+
+// The residual on 1D factors.  Same work mapping, shapes and epilogue as
+// dg_residual_kernel, which needs U (F + D U) + F U multiply-adds per velocity
+// and element with every matrix entry a constant of its own (p = 3: 1,024 and
+// 4 KB); the factors need 4 n^2 (traces) + 2 n^3 (derivative) + 4 n^2 (traces
+// of the transformed flux) + 8 n^2 (lift) (p = 3: 384, 48 constants), so the
+// loads bound the kernel instead of the instructions.  Boundary and halo flux
+// points are evaluated in a loop over the lane's own ones before the flux work
+// (its code once, not once per flux point); interior warps skip it.
+template <typename T, int n, int VPT, int PF, int MB>
+__global__ void __launch_bounds__(256, MB) dg_residual_fac_kernel(const DgArgs<T> a, const DgFac<T, n> op) {
+  constexpr int U = n * n, F = 4 * n, D = 2;
+  using G = DgGeo<T, U, F, D>;
+  __shared__ __align__(16) T sg[32 * G::GS];
+  __shared__ __align__(16) int64_t sp[32 * G::PS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  {
+    const T* gs = a.geoblk + (size_t)blockIdx.x * 32 * G::GS;
+    for (int i = threadIdx.x; i < 32 * G::GS; i += 256) sg[i] = gs[i];
+    const int64_t* ps = a.pblk + (size_t)blockIdx.x * 32 * G::PS;
+    for (int i = threadIdx.x; i < 32 * G::PS; i += 256) sp[i] = ps[i];
+  }
+  __syncthreads();
+  const int64_t e = (int64_t)blockIdx.x * 32 + lane;
+  if (e >= a.neles) return;
+  const T* gl = sg + lane * G::GS;
+  const int64_t* pl = sp + lane * G::PS;
+  const int vend = a.v0 + a.nv;
+  const int vbeg = a.v0 + (int)blockIdx.y * (8 * VPT) + w;
+  unsigned bmask = 0;  // flux points whose partner is not an element of this part
+#pragma unroll
+  for (int f = 0; f < F; ++f) bmask |= pl[f] < 0 ? 1u << f : 0u;
+
+#pragma unroll 1
+  for (int it = 0; it < VPT; ++it) {
+    const int v = vbeg + 8 * it;
+    if (v >= vend) break;
+    const int64_t o = ((int64_t)blockIdx.x * a.V + v) * 32 + lane;
+
+    // every bank value of this (v, e) first, so the loads overlap
+    T u[U];
+    {
+      const T* up = a.u + o;
+#pragma unroll
+      for (int i = 0; i < U; ++i, up += a.ldim_u) u[i] = __ldg(up);
+    }
+    T K[PF ? U : 1];
+    if constexpr (PF != 0) {
+#pragma unroll
+      for (int r = 0; r < U; ++r) {
+        const int64_t ro = o + (int64_t)r * a.ldim_u;
+        T k = a.Cq ? a.gamma * __ldg(a.Cq + ro) : T(0);
+        if (a.A) k = fma(a.alpha, __ldg(a.A + ro), k);
+        if (a.B) k = fma(a.beta, __ldg(a.B + ro), k);
+        K[r] = k;
+      }
+    }
+    // the face values come from the interp kernel: wait for it (returns at
+    // once after the first iteration)
+    pdl_wait();
+    T urv[F];
+#pragma unroll
+    for (int f = 0; f < F; f += 2) {
+      const longlong2 pb = reinterpret_cast<const longlong2*>(pl)[f / 2];
+      urv[f] = pb.x >= 0 ? a.uf[pb.x + (int64_t)v * 32] : T(0);
+      urv[f + 1] = pb.y >= 0 ? a.uf[pb.y + (int64_t)v * 32] : T(0);
+    }
+    const T c[3] = {__ldg(a.cvx + v), __ldg(a.cvy + v), __ldg(a.cvz + v)};
+    unsigned omask = 0;  // boundary points whose ghost value is the interior one
+    if (bmask) {
+      for (unsigned m = bmask; m; m &= m - 1) {
+        const int f = __ffs(m) - 1, b = (int)(-pl[f] - 1);
+        T val = T(0);
+        if (b >= a.nb) {
+          val = a.halo[(int64_t)(b - a.nb) * a.V + v];
+        } else {
+          const T nmv[D] = {gl[G::ON + f * D], gl[G::ON + f * D + 1]};
+          if (dg_ghost<T, D>(a, b, v, e, f, c, nmv, &val)) omask |= 1u << f;
+        }
+#pragma unroll
+        for (int g = 0; g < F; ++g) urv[g] = g == f ? val : urv[g];
+      }
+    }
+
+    // transformed flux at the solution points F~_(i,k) = (sum_kk S_ik,kk c_kk) u_k
+    T fx[U], fe[U];
+    if constexpr (G::VW == 4) {
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        T sm[4];
+        lds16<T, 1>(gl + G::OS + 4 * k, sm);
+        fx[k] = fma(sm[1], c[1], sm[0] * c[0]) * u[k];
+        fe[k] = fma(sm[3], c[1], sm[2] * c[0]) * u[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        T sm[4];
+        lds16<T, 2>(gl + G::OS + 4 * k, sm);
+        fx[k] = fma(sm[1], c[1], sm[0] * c[0]) * u[k];
+        fe[k] = fma(sm[3], c[1], sm[2] * c[0]) * u[k];
+      }
+    }
+    // common normal flux |S^T n| F^ at flux point f (rusanov.mako:46-50 with
+    // the scaled normal), ul the interior trace
+    auto common = [&](int f, T ul) -> T {
+      const T nc = fma(gl[G::ON + f * D + 1], c[1], gl[G::ON + f * D] * c[0]);
+      const T ur = omask >> f & 1 ? ul : urv[f];
+      return T(0.5) * nc * (ul + ur) + T(0.5) * fabs(nc) * (ul - ur);
+    };
+    T R[U];
+    // along xi (faces 3 and 1), then along eta (faces 0 and 2): the derivative
+    // and the lift of the jump between common and interior normal flux
+    {
+      T j0[n], j1[n];
+#pragma unroll
+      for (int t = 0; t < n; ++t) {
+        T ul0 = op.l[0][0] * u[t * n], ul1 = op.l[1][0] * u[t * n];
+        T g0 = op.l[0][0] * fx[t * n], g1 = op.l[1][0] * fx[t * n];
+#pragma unroll
+        for (int i = 1; i < n; ++i) {
+          ul0 = fma(op.l[0][i], u[t * n + i], ul0);
+          ul1 = fma(op.l[1][i], u[t * n + i], ul1);
+          g0 = fma(op.l[0][i], fx[t * n + i], g0);
+          g1 = fma(op.l[1][i], fx[t * n + i], g1);
+        }
+        j0[t] = common(3 * n + t, ul0) + g0;
+        j1[t] = common(n + t, ul1) - g1;
+      }
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        T h0 = op.la[j][0] * j0[0], h1 = op.la[j][0] * j1[0];
+#pragma unroll
+        for (int t = 1; t < n; ++t) {
+          h0 = fma(op.la[j][t], j0[t], h0);
+          h1 = fma(op.la[j][t], j1[t], h1);
+        }
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          T s = fma(op.lc[1][i], h1, op.lc[0][i] * h0);
+#pragma unroll
+          for (int k = 0; k < n; ++k) s = fma(op.d[i][k], fx[j * n + k], s);
+          R[j * n + i] = s;
+        }
+      }
+    }
+    {
+      T j0[n], j1[n];
+#pragma unroll
+      for (int t = 0; t < n; ++t) {
+        T ul0 = op.l[0][0] * u[t], ul1 = op.l[1][0] * u[t];
+        T g0 = op.l[0][0] * fe[t], g1 = op.l[1][0] * fe[t];
+#pragma unroll
+        for (int i = 1; i < n; ++i) {
+          ul0 = fma(op.l[0][i], u[i * n + t], ul0);
+          ul1 = fma(op.l[1][i], u[i * n + t], ul1);
+          g0 = fma(op.l[0][i], fe[i * n + t], g0);
+          g1 = fma(op.l[1][i], fe[i * n + t], g1);
+        }
+        j0[t] = common(t, ul0) + g0;
+        j1[t] = common(2 * n + t, ul1) - g1;
+      }
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        T h0 = op.la[i][0] * j0[0], h1 = op.la[i][0] * j1[0];
+#pragma unroll
+        for (int t = 1; t < n; ++t) {
+          h0 = fma(op.la[i][t], j0[t], h0);
+          h1 = fma(op.la[i][t], j1[t], h1);
+        }
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+          T s = fma(op.lc[1][j], h1, fma(op.lc[0][j], h0, R[j * n + i]));
+#pragma unroll
+          for (int k = 0; k < n; ++k) s = fma(op.d[j][k], fe[k * n + i], s);
+          R[j * n + i] = s;
+        }
+      }
+    }
+
+    const T* const rj = gl + G::OR;
     if constexpr (PF != 0) {
       T* op_ = a.out + o;
 #pragma unroll

@@ -172,7 +172,8 @@ __global__ void __launch_bounds__(128, MB)
         const int64_t pb = pl[f];
         if (pb < 0) {
           const int b = (int)(-pb - 1);
-          ur = b >= a.nb ? a.halo[(int64_t)(b - a.nb) * a.V + v] : dg_ghost<float, D>(a, b, v, e, f, c, nmv, nc, ul);
+          if (b >= a.nb) ur = a.halo[(int64_t)(b - a.nb) * a.V + v];
+          else if (dg_ghost<float, D>(a, b, v, e, f, c, nmv, &ur)) ur = ul;
         }
         phi[f] = 0.5f * nc * (ul + ur) + 0.5f * fabsf(nc) * (ul - ur);  // rusanov.mako:46-50
       }

@@ -70,6 +70,7 @@ _lib.declare('dgfs_dg_num_variants', c_int, [c_void_p, c_ip])
 _lib.declare('dgfs_dg_variant_info', c_int, [c_void_p, c_int, c_ip, c_ip,
                                              c_ip])
 _lib.declare('dgfs_dg_select', c_int, [c_void_p, c_int])
+_lib.declare('dgfs_dg_selected', c_int, [c_void_p, c_ip])
 _lib.declare('dgfs_dg_variant_tc', c_int, [c_void_p, c_int, c_ip])
 _lib.declare('dgfs_dg_status', c_int, [c_void_p, c_void_p, c_ip])
 _lib.declare('dgfs_dg_bcvals', c_int, [c_void_p, c_dp, c_int])
@@ -167,7 +168,6 @@ class DGFSSystem:
         self.surrogate = None
         self.collide_hook = None
         self.halo_exchange = halo_exchange
-        self._dg_shape = 0
         self._build_dg()
 
     # -- DG handle ----------------------------------------------------------
@@ -290,6 +290,9 @@ class DGFSSystem:
         _lib.check(lib.dgfs_dg_create(ct.byref(p), ct.byref(h)),
                    'dgfs_dg_create')
         self._dg, self._lib = h, lib
+        idx = c_int()
+        _lib.check(lib.dgfs_dg_selected(h, ct.byref(idx)), 'dgfs_dg_selected')
+        self._dg_shape = idx.value
         if self.halo is not None:
             import torch
             tdt = torch.float64 if self.backend.precision == 64 else \

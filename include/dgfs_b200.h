@@ -361,11 +361,13 @@ DGFS_API int dgfs_dg_invmass(dgfs_dg* h, const void* u, void* out, int v0,
  * index the velocities per warp, whether the Runge-Kutta terms are loaded
  * ahead of the flux work, and the CTAs per SM the register budget was
  * compiled for; dgfs_dg_select sets the shape of later dgfs_dg_rhs calls
- * (index 0 by default).  No counterpart in the reference. */
+ * (by default the one dgfs_dg_create picks for the mesh's size;
+ * dgfs_dg_selected tells which).  No counterpart in the reference. */
 DGFS_API int dgfs_dg_num_variants(const dgfs_dg* h, int* count);
 DGFS_API int dgfs_dg_variant_info(const dgfs_dg* h, int idx, int* vpt,
                                   int* prefetch, int* min_ctas_per_sm);
 DGFS_API int dgfs_dg_select(dgfs_dg* h, int idx);
+DGFS_API int dgfs_dg_selected(const dgfs_dg* h, int* idx);
 /* 1 when shape idx runs the element-operator contraction on the tensor
  * cores (FP32 handles: tcgen05.mma kind::tf32 with operands split into
  * two TF32 parts, FP32 accuracy), 0 for the SIMT shapes. */
