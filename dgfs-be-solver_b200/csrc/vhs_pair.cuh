@@ -36,11 +36,14 @@
 // a warp is one plane k1, so the first two passes need no barrier at all
 // between them (N = 24: groups of 4 planes, 3 warps).  The third pass releases
 // the work cube as soon as its values are in registers.  NQ more threads
-// transform the Nyquist planes (one line each).
-// Measured on one B200: FP32 N = 32 (16 x 24 (p, q)), 2,592 points: 112.4 ms a
-// sweep against 140.5 ms for the scalar-transform form (116.8 ms with the
-// Nyquist lines on main threads); FP64 N = 24, 576 points: 10.98 ms against
-// 15.05 ms (12.19 ms).
+// transform the Nyquist planes (one line each).  The Nyquist products, which
+// need only the CTA's own tables, are added while the halves travel.
+// Measured on one B200: FP32 N = 32 (16 x 24 (p, q)), 2,592 points: 109.9 ms a
+// sweep against 140.5 ms for the scalar-transform form (112.4 ms with the
+// Nyquist products after the third pass, 113.6 ms with the Nyquist lines on
+// main threads); FP64 N = 24, 576 points: 10.53 ms against 15.05 ms (10.98,
+// 11.82 ms).  Handing over by one thread's cluster-scope mbarrier arrivals after
+// a CTA barrier, instead of the cluster barrier, measured 120.4 and 11.79 ms.
 //
 // Shared memory (complex): W [MH][N][N + 1], the Nyquist planes T1 [x2 in
 // X_r][x3], T2 [x1][x3], T3 [x2 in X_r][x1], F^ on them [k][line] and their
@@ -108,19 +111,6 @@ __device__ __forceinline__ void cl_sync() {
   cl_wait();
 }
 
-// third-pass line (x2l = hi, x3 = lo) along k1: the k1 of this CTA from its
-// work cube (row kinv(k1) N + x2, x2 = MH r + hi), the others from the
-// peer's staging buffer ([kinv(k1)][hi][lo], written before the barrier)
-template <typename T, int N>
-__device__ __forceinline__ void pair_load3(cx<T> (&x)[N], const cx<T>* sW, const cx<T>* xpeer, int r, int hi,
-                                           int lo) {
-  constexpr int LP = N + 1, MH = N / 2;
-#pragma unroll
-  for (int k1 = 0; k1 < N; ++k1)
-    x[k1] = pair_owner<N>(k1) == r ? sW[(pair_kinv<N>(k1) * N + MH * r + hi) * LP + lo]
-                                   : __ldcg(xpeer + (pair_kinv<N>(k1) * MH + hi) * N + lo);
-}
-
 template <typename T, int NV, bool OWN>
 __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(const VhsArgs<T> a) {
   using G = PairGeom<T, NV, OWN>;
@@ -128,7 +118,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
   using CM = cx<T>;  // in the tables and the scratch
   constexpr int N = G::N, NY = G::NY, NN = G::NN, V = G::V, LP = G::LP, NM = G::NM, MH = G::MH, Q = G::Q;
   constexpr int NT = G::NT, GT = G::GT, PHS = G::PHS, WD = G::WD;
-  constexpr int B_T = 1, B_G = 2;  // named barriers: Nyquist tables, groups
+  constexpr int B_T = 1, B_N = 2, B_G = 3;  // named barriers: old and new Nyquist tables, groups
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const base = reinterpret_cast<C*>(smem_raw);
@@ -414,18 +404,40 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           }
           group_sync();
           pass2_out();
-          cl_sync();            // both halves staged, the Nyquist tables complete
-          // pass 3: lines (x2, x3) along k1; S += Re P Im P + Re Nq Im Nq
+          cl_arrive();
+          // While the halves travel: S += Re Nq Im Nq on this thread's
+          // third-pass line, Nq = s1 T1(x2, x3) + s2 T2(x1, x3) + s3 T3(x1, x2)
+          // with s = (-1)^x (a common sign drops out: s3 Nq is formed)
+          bar_sync(B_N, NT);    // the Nyquist tables are complete
+          constexpr int SC = 8;  // values per step
+          tmem_store_wait();
+          {
+            const T s3 = (lo & 1) ? T(-1) : T(1), s23 = (x2 & 1) ? -s3 : s3;
+            const C t1 = vmul(sT1[tid], vmk(s3, s3)), ss = vmk(s23, s23);
+            sfor<0, N / SC>([&](auto cc) {
+              constexpr int c = decltype(cc)::value;
+              uint32_t t[SC * WD];
+              tm_load(tmS + SC * c * WD, t);
+              tm_wait(t);
+#pragma unroll
+              for (int h = 0; h < SC; ++h) {
+                const int i = SC * c + h;
+                const C u = sT3[hi * LP + i];
+                const C n = vfma(sT2[i * N + lo], ss, (i & 1) ? vsub(u, t1) : vadd(u, t1));
+                tm_put(t, h, fma(cre(n), cim(n), q == 0 ? T(0) : tm_get(t, h, T(0))));
+              }
+              tm_store(tmS + SC * c * WD, t);
+            });
+          }
+          cl_wait();            // both halves staged
+          // pass 3: lines (x2, x3) along k1; S += Re P Im P
           C x[N];
           load3(x);
           __syncwarp();
           if (tid % 32 == 0) mbar_arrive(&s_read);  // this warp's part of the cube may be overwritten
           rphase ^= 1;
-          tmem_store_wait();
           cfft<N, 1>(x);
-          const T s3 = (lo & 1) ? T(-1) : T(1), s23 = (x2 & 1) ? -s3 : s3;
-          const C t1 = vmul(sT1[tid], vmk(s3, s3)), ss = vmk(s23, s23);
-          constexpr int SC = 8;  // values per step
+          tmem_store_wait();
           sfor<0, N / SC>([&](auto cc) {
             constexpr int c = decltype(cc)::value;
             uint32_t t[SC * WD];
@@ -433,11 +445,8 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
             tm_wait(t);
 #pragma unroll
             for (int h = 0; h < SC; ++h) {
-              const int i = SC * c + h;
-              const C u = sT3[hi * LP + i];
-              const C n = vfma(sT2[i * N + lo], ss, (i & 1) ? vsub(u, t1) : vadd(u, t1));
-              const T s0 = q == 0 ? T(0) : tm_get(t, h, T(0));
-              tm_put(t, h, fma(cre(x[i]), cim(x[i]), fma(cre(n), cim(n), s0)));
+              const C v = x[SC * c + h];
+              tm_put(t, h, fma(cre(v), cim(v), tm_get(t, h, T(0))));
             }
             tm_store(tmS + SC * c * WD, t);
           });
@@ -512,6 +521,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           slot ^= 1;
           bar_sync(B_T, NT);  // every first axis is done, and no main thread reads the old tables
           nyq_second();
+          bar_arrive(B_N, NT);
           cl_sync();
         }
         cl_sync();
