@@ -144,8 +144,11 @@ struct dgfs_vss {
   int max_clusters;
   void* phase;  // cx<T> [P][M][2][3][N]
   void* b;      // cx<T> [P][M][V], weight w_x folded in
+  void* bt;     // ... with the last axis outermost, where the two-CTA kernel exists
+                // (b is then made from it if the push kernel is selected)
   void* phase_h;  // cx<T> [P][Mh][2][3][N] (Mh > 0)
   void* b_h;      // cx<T> [P][Mh][V]: b(y) + b(-y)
+  void* bt_h;     // ... with the last axis outermost
   void* c;      // cx<T> [V]
   void* fc;     // scratch: [clusters * C][V / C] cx<T> (push), per pair (two-CTA)
   size_t fc_bytes;
@@ -232,6 +235,10 @@ template <typename T> int build(dgfs_vss* h, const dgfs_vss_params* p) {
   std::vector<int> all(M);
   for (int y = 0; y < M; ++y) all[y] = y;
 
+  // the two-CTA kernel, where it exists, takes the gain kernels with the last
+  // axis outermost (its lanes, one line (k1, k2) each, read consecutive
+  // entries); the push kernel's order is made from it if that is selected
+  const bool two_cta = vss_shape(h->prec, N, 1) != nullptr;
   // axis phases [P][K][2][3][N] and weighted gain kernels [P][K][V] of the
   // directions `dirs` (each with its antipode's b added when `pairs`)
   std::vector<std::complex<double>> eb((size_t)Mp * V), row(V);
@@ -262,7 +269,11 @@ template <typename T> int build(dgfs_vss* h, const dgfs_vss_params* p) {
             const std::complex<double>* e = eb.data() + (size_t)y2 * V;
             for (int v = 0; v < V; ++v) row[v] += bb * e[v];
           }
-          for (int v = 0; v < V; ++v) dst[v] += row[v] * (w * fac_b);
+          if (two_cta)  // last axis outermost
+            for (int k = 0; k < N; ++k)
+              for (int l = 0; l < N * N; ++l) dst[(size_t)k * N * N + l] += row[(size_t)l * N + k] * (w * fac_b);
+          else
+            for (int v = 0; v < V; ++v) dst[v] += row[v] * (w * fac_b);
         }
       }
     }
@@ -287,12 +298,13 @@ template <typename T> int build(dgfs_vss* h, const dgfs_vss_params* p) {
   std::vector<std::complex<double>> phase, b;
   tables(all, false, phase, b);
   int rc;
-  if ((rc = upload_cx<T>(&h->phase, phase)) || (rc = upload_cx<T>(&h->b, b)) || (rc = upload_cx<T>(&h->c, c)))
+  if ((rc = upload_cx<T>(&h->phase, phase)) || (rc = upload_cx<T>(two_cta ? &h->bt : &h->b, b)) ||
+      (rc = upload_cx<T>(&h->c, c)))
     return rc;
   h->Mh = 0;
   if (halve) {
     tables(rep, true, phase, b);
-    if ((rc = upload_cx<T>(&h->phase_h, phase)) || (rc = upload_cx<T>(&h->b_h, b))) return rc;
+    if ((rc = upload_cx<T>(&h->phase_h, phase)) || (rc = upload_cx<T>(two_cta ? &h->bt_h : &h->b_h, b))) return rc;
     h->Mh = (int)rep.size();
   }
   return DGFS_OK;
@@ -304,6 +316,8 @@ void free_vss(dgfs_vss* h) {
   cudaFree(h->b);
   cudaFree(h->phase_h);
   cudaFree(h->b_h);
+  cudaFree(h->bt);
+  cudaFree(h->bt_h);
   cudaFree(h->c);
   cudaFree(h->fc);
   cudaFree(h->err);
@@ -313,6 +327,36 @@ void free_vss(dgfs_vss* h) {
 }  // namespace
 
 namespace {
+
+// [.][k3][k1 k2] -> [.][k1 k2][k3], one block per (direction, 32 lines)
+__global__ void untranspose_kernel(const float2* __restrict__ in, float2* __restrict__ out, int N) {
+  const int NN = N * N, l = blockIdx.x * 32 + threadIdx.x;
+  const size_t d = (size_t)blockIdx.y * NN * N;
+  if (l >= NN) return;
+  for (int k = threadIdx.y; k < N; k += blockDim.y) out[d + (size_t)l * N + k] = in[d + (size_t)k * NN + l];
+}
+
+// The push kernel's gain-kernel tables of a handle built for the two-CTA
+// kernel (set-up: allocates and synchronises).
+int make_push_tables(dgfs_vss* h) {
+  struct {
+    void* in;
+    void** out;
+    int dirs;
+  } t[2] = {{h->bt, &h->b, h->P * h->M}, {h->bt_h, &h->b_h, h->P * h->Mh}};
+  for (auto& e : t) {
+    if (!e.in || *e.out) continue;
+    if (cudaMalloc(e.out, (size_t)e.dirs * h->V * sizeof(float2)) != cudaSuccess) {
+      *e.out = nullptr;
+      return set_error(DGFS_ERR_NOMEM, "gain-kernel table allocation failed");
+    }
+    untranspose_kernel<<<dim3((h->N * h->N + 31) / 32, e.dirs), dim3(32, 8)>>>((const float2*)e.in, (float2*)*e.out,
+                                                                               h->N);
+  }
+  if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+    return set_error(DGFS_ERR_CUDA, "gain-kernel tables: %s", cudaGetErrorString(cudaGetLastError()));
+  return DGFS_OK;
+}
 
 // Kernel attributes, the clusters that fit the device and the scratch of a
 // launch shape (the scratch grows, never shrinks).
@@ -470,6 +514,7 @@ extern "C" int dgfs_vss_apply(dgfs_vss* h, const void* fp, const void* fq, void*
     a.M = half ? h->Mh : h->M;
     a.phase = (const float2*)(half ? h->phase_h : h->phase);
     a.b = (const float2*)(half ? h->b_h : h->b);
+    a.bt = (const float2*)(half ? h->bt_h : h->bt);
     a.c = (const float2*)h->c;
     a.fc = (float2*)h->fc;
     a.err = h->err;
@@ -488,6 +533,10 @@ extern "C" int dgfs_vss_select(dgfs_vss* h, int pair) {
   if (!shape)
     return set_error(DGFS_ERR_UNSUPPORTED, "no %s VSS kernel for Nv=%d precision=%d", pair ? "two-CTA" : "cluster",
                      h->N, h->prec);
+  if (!shape->pair) {
+    const int rc = make_push_tables(h);
+    if (rc) return rc;
+  }
   return set_shape(h, shape);
 }
 

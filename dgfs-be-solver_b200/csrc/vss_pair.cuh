@@ -19,13 +19,22 @@
 // of every line it owns in x2 (a staging buffer in the L2 scratch, one
 // cluster barrier), and runs along k1 on the lines (x2 in X_r, x3).  The
 // forward transform of g h runs the other way: along x1, the hand-over of
-// the k1 the other CTA owns, along x2, along x3; the gain spectrum QGhat
-// of the CTA's k-slab accumulates in shared memory.
+// the k1 the other CTA owns, along x2, along x3.
 //
 // 576 threads: 288 take the g field's lines and 288 the h field's (one line
-// each per pass); the forward transform of g h uses the first 288.
-// Shared memory (complex float): Wg, Wh [MH][N][N+1], QGhat [N][MH][N]
-// (k3, k1l, k2), two phase slots [2 fields][3][N]: 174 KB.
+// each per pass, packed FP32 transforms, fft_vec.cuh); the forward transform
+// of g h uses the first 288, beside which the h threads already run the first
+// two passes of the next direction.  Each thread's spectrum line and, for the
+// first 288, the gain spectrum QGhat of line (k1, k2) live in tensor memory; a
+// second pass waits for its group of 4 planes only.  What bounds it is the
+// chain of six passes and two cluster barriers per direction.  Measured on one
+// B200 (N = 24, 12 x 32 directions, four ordered pairs, 144 points): 25.3 ms
+// against 32.7 ms with the spectra read from L2, QGhat in shared memory, scalar
+// transforms and every pass behind a CTA barrier.  Handing over by one thread's
+// cluster-scope mbarrier arrivals, with the two fields' chains decoupled,
+// measured 25.1 ms and was not kept.
+// Shared memory (complex float): Wg, Wh [MH][N][N+1], the h field after its
+// third pass [x1][line], two phase slots [2 fields][3][N]: 173 KB.
 #pragma once
 
 #include "vhs_pair.cuh"
@@ -38,78 +47,108 @@ template <int N_> struct VssPairGeom {
   static constexpr int MH = N / 2, LP = N + 1;
   static constexpr int NL = MH * N;                  // lines of a pass and field
   static constexpr int NT = 2 * NL;                  // threads: a g line and an h line each
+  static constexpr int GT = 4 * N;                   // threads of a group of 4 planes
   static constexpr int WSZ = MH * N * LP;            // cx per work cube
-  static constexpr int OFF_WG = 0, OFF_WH = WSZ, OFF_QG = 2 * WSZ;
-  static constexpr int OFF_PH = OFF_QG + N * MH * N;  // [2 slots][2 fields][3][N]
+  static constexpr int OFF_WG = 0, OFF_WH = WSZ, OFF_SH = 2 * WSZ;
+  static constexpr int OFF_PH = OFF_SH + N * NL;     // [2 slots][2 fields][3][N]
   static constexpr int SMEM_CX = OFF_PH + 2 * 6 * N;
   static constexpr int SLICE = H * NN;               // half spectrum in the scratch
   static constexpr int XSLAB = MH * MH * N;          // staging buffer [k1l][j][x3]
-  // scratch per pair: F, G, [2 CTAs][2 alternating buffers][2 fields] staging
-  static constexpr int SCRATCH = 2 * SLICE + 8 * XSLAB;
-  static_assert(NT % 32 == 0 && NT <= 1024, "thread layout");
+  // scratch per pair: F, G, staging of the inverse transforms [2 CTAs][2
+  // alternating][2 fields] and of the forward one [2 CTAs][2]
+  static constexpr int SCRATCH = 2 * SLICE + 12 * XSLAB;
+  static constexpr int TW = 4 * N;                   // tensor memory columns per warp: line, QGhat
+  static constexpr int TCOLS = 512;
+  static_assert(NT % 32 == 0 && NL % 32 == 0 && GT % 32 == 0 && NL % GT == 0 && NT <= 1024, "thread layout");
+  static_assert((NT / 32 + 3) / 4 * TW <= TCOLS, "tensor memory");
 };
-
-// Second pass of an inverse transform: the line (k1l = hi, x3 = lo) of a
-// work cube W along k2; the outputs with x2 in X_r stay in W, the others go
-// to the staging buffer xs for the peer ([k1l][x2 - MH (1 - r)][x3]).
-template <int N>
-__device__ __forceinline__ void vss_pair_pass2(cx<float>* sW, cx<float>* xs, int r, int hi, int lo) {
-  constexpr int LP = N + 1, MH = N / 2;
-  cx<float> x[N];
-#pragma unroll
-  for (int j = 0; j < N; ++j) x[j] = sW[(hi * N + j) * LP + lo];
-  fft<float, N, +1>(x);
-#pragma unroll
-  for (int j = 0; j < MH; ++j) {
-    sW[(hi * N + MH * r + j) * LP + lo] = r ? x[MH + j] : x[j];
-    __stcg(xs + (hi * MH + j) * N + lo, r ? x[j] : x[MH + j]);
-  }
-}
 
 template <int N>
 __global__ void __launch_bounds__(VssPairGeom<N>::NT, 1) vss_pair_kernel(const VssArgs<float> a) {
   using G = VssPairGeom<N>;
-  using C = cx<float>;
-  constexpr int H = G::H, NY = G::NY, NN = G::NN, V = G::V, LP = G::LP, MH = G::MH, NL = G::NL;
+  using C = cpx;
+  using CM = float2;
+  constexpr int H = G::H, NY = G::NY, NN = G::NN, V = G::V, LP = G::LP, MH = G::MH, NL = G::NL, GT = G::GT;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* const sWg = reinterpret_cast<C*>(smem_raw) + G::OFF_WG;
-  C* const sWh = reinterpret_cast<C*>(smem_raw) + G::OFF_WH;
-  C* const sQG = reinterpret_cast<C*>(smem_raw) + G::OFF_QG;
-  C* const sPh = reinterpret_cast<C*>(smem_raw) + G::OFF_PH;
+  C* const base = reinterpret_cast<C*>(smem_raw);
+  CM* const sPh = reinterpret_cast<CM*>(base + G::OFF_PH);
+  __shared__ uint32_t s_tmem;
 
   cg::cluster_group cluster = cg::this_cluster();
   const int r = (int)cluster.block_rank();
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, wid = tid / 32;
   // field of this thread (0: g from F, 1: h from G) and its line in a pass:
   // hi = L / N (k1l, or x2l in the third pass), lo = L % N (k2, x3)
   const int fld = tid / NL, L = tid % NL, hi = L / N, lo = L % N;
-  C* const sW = fld ? sWh : sWg;
+  const int k1 = pair_kmap<N>(r, hi), x2 = MH * r + hi;
+  C* const sW = base + (fld ? G::OFF_WH : G::OFF_WG);
+  C* const w1p = sW + L * LP;               // line (k1l, k2) along k3
+  C* const w2p = sW + hi * N * LP + lo;     // line (k1l, x3) along k2
+  C* const w3p = sW + x2 * LP + lo;         // line (x2, x3) along k1l: stride N LP
+  C* const sH = base + G::OFF_SH + L;       // h of line L: stride NL
   const int cid = blockIdx.x / 2, ncl = gridDim.x / 2;
-  C* const Fg = a.fc + (size_t)cid * G::SCRATCH;
-  C* const Gg = Fg + G::SLICE;
-  C* const Xs = Gg + G::SLICE;  // staging: [rank][buffer][field][k1l][j][x3]
-  const float invV = 1.f / (float)V;
+  CM* const Fg = a.fc + (size_t)cid * G::SCRATCH;
+  CM* const Gg = Fg + G::SLICE;
+  CM* const Xi = Gg + G::SLICE + fld * G::XSLAB + lo;  // inverse staging [rank][parity][field][k1l][j][x3]
+  CM* const Xf = Gg + G::SLICE + 8 * G::XSLAB + lo;    // forward staging [rank][parity][k1l][x2l][x3]
   const int npq = a.P * a.M;
-  int xb = 0;  // staging buffer of the next exchange
-  auto xmine = [&](int b, int f) { return Xs + (size_t)((r * 2 + b) * 2 + f) * G::XSLAB; };
-  auto xpeer = [&](int b, int f) { return (const C*)(Xs + (size_t)(((r ^ 1) * 2 + b) * 2 + f) * G::XSLAB); };
   // a spectrum value at (k1, k2, k3) from a half spectrum in the scratch
-  auto at = [&](const C* S, int k1, int k2, int k3) -> C {
-    if (k3 <= NY) return __ldcg(S + (k3 * N + k1) * N + k2);
-    const C c = __ldcg(S + ((N - k3) * N + (N - k1) % N) * N + (N - k2) % N);
-    return mk<C>(c.x, -c.y);
+  auto at = [&](const CM* S, int i1, int i2, int i3) -> C {
+    if (i3 <= NY) return from_c(__ldcg(S + (i3 * N + i1) * N + i2));
+    const CM c = __ldcg(S + ((N - i3) * N + (N - i1) % N) * N + (N - i2) % N);
+    return vmk(c.x, -c.y);
   };
+  auto group_sync = [&]() { bar_sync(1 + tid / GT, GT); };
 
-  // Second pass of an inverse transform (vss_pair_pass2) and the exchange;
-  // returns the staging buffer to read.
-  auto inverse_pass2 = [&]() -> int {
-    vss_pair_pass2<N>(sW, xmine(xb, fld), r, hi, lo);
-    cl_arrive();
-    cl_wait();  // both halves staged (cluster-scope release / acquire)
-    const int b = xb;
-    xb ^= 1;
-    return b;
+  if (tid < 32) tmem_alloc(&s_tmem, G::TCOLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmF = s_tmem + ((uint32_t)(wid % 4 * 32) << 16) + wid / 4 * G::TW, tmQ = tmF + 2 * N;
+
+  // first pass of an inverse transform is in the work cube: the second pass
+  // (lines (k1l, x3) along k2) of exchange `par`; outputs with x2 in X_r stay
+  // in the cube, the others go to the staging buffer
+  auto pass2_out = [&](int par) {
+    group_sync();
+    C x[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = w2p[j * LP];
+    cfft<N, 1>(x);
+    CM* const xs = Xi + (r * 2 + par) * 2 * G::XSLAB + hi * MH * N;
+#pragma unroll
+    for (int j = 0; j < MH; ++j) {
+      w2p[(MH * r + j) * LP] = r ? x[MH + j] : x[j];
+      __stcg(xs + j * N, to_c(r ? x[j] : x[MH + j]));
+    }
+  };
+  // passes 1 and 2 of direction pq's field
+  auto inverse12 = [&](int pq) {
+    const CM* ph = sPh + (pq & 1) * 6 * N + fld * 3 * N;
+    const CM e12 = cmul(ph[k1], ph[N + lo]);
+    uint32_t t[2 * N];
+    tm_load(tmF, t);
+    tm_wait(t);
+    C x[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const CM e = cmul(e12, ph[2 * N + k]);
+      const float re = tm_get(t, 2 * k, 0.f), im = tm_get(t, 2 * k + 1, 0.f);
+      x[k] = vmk(re * e.x - im * e.y, re * e.y + im * e.x);
+    }
+    cfft<N, 1>(x);
+#pragma unroll
+    for (int k = 0; k < N; ++k) w1p[k] = x[k];
+    pass2_out(pq & 1);
+  };
+  // third-pass line along k1: this CTA's planes from the cube, the others
+  // from the peer's staging buffer
+  auto load3 = [&](C (&x)[N], int par) {
+    const CM* const xp = Xi + ((r ^ 1) * 2 + par) * 2 * G::XSLAB + hi * N;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      x[k] = pair_owner<N>(k) == r ? w3p[pair_kinv<N>(k) * N * LP] : from_c(__ldcg(xp + pair_kinv<N>(k) * MH * N));
   };
 
 #pragma unroll 1
@@ -119,33 +158,32 @@ __global__ void __launch_bounds__(VssPairGeom<N>::NT, 1) vss_pair_kernel(const V
 
     // ---- F = FFT(f_p) / V (field 0) and G = FFT(f_q) / V (field 1) -------
     // lines (x1 = MH r + hi, x2 = lo) along x3, then (x1l, k3) along x2,
-    // through the staging buffers, then (k2, k3) along x1
+    // through the scratch, then (k2, k3) along x1
     {
       const float* f = fld ? a.fq : a.fp;
       const int64_t b0 = soa_ix(upt, a.ldim, elem, (int64_t)((MH * r + hi) * N + lo) * N, V, a.soasz);
       C x[N];
 #pragma unroll
-      for (int k = 0; k < N; ++k) x[k] = mk<C>(f[b0 + (int64_t)k * a.soasz], 0.f);
-      fft<float, N, -1>(x);
+      for (int k = 0; k < N; ++k) x[k] = vmk(f[b0 + (int64_t)k * a.soasz], 0.f);
+      cfft<N, -1>(x);
 #pragma unroll
-      for (int k = 0; k <= NY; ++k) sW[(hi * N + lo) * LP + k] = x[k];
+      for (int k = 0; k <= NY; ++k) w1p[k] = x[k];
     }
     __syncthreads();
     // exchange buffer [k3][x1][k2] of each field: the half spectrum slot
     // itself (written by both CTAs, each its x1 half)
-    C* const S = fld ? Gg : Fg;
+    CM* const S = fld ? Gg : Fg;
 #pragma unroll 1
     for (int t = L; t < MH * H; t += NL) {
       const int x1l = t / H, k3 = t % H;
       C x[N];
 #pragma unroll
       for (int j = 0; j < N; ++j) x[j] = sW[(x1l * N + j) * LP + k3];
-      fft<float, N, -1>(x);
+      cfft<N, -1>(x);
 #pragma unroll
-      for (int j = 0; j < N; ++j) __stcg(S + (k3 * N + MH * r + x1l) * N + j, x[j]);
+      for (int j = 0; j < N; ++j) __stcg(S + (k3 * N + MH * r + x1l) * N + j, to_c(x[j]));
     }
-    cl_arrive();
-    cl_wait();  // every x1 of both fields in the scratch
+    cl_sync();  // every x1 of both fields in the scratch
     // lines (k2 in this CTA's half, k3) along x1, into registers, then
     // back in place once both CTAs have read (a second barrier)
     C y[N];
@@ -153,142 +191,150 @@ __global__ void __launch_bounds__(VssPairGeom<N>::NT, 1) vss_pair_kernel(const V
     const int k2f = MH * r + (fwd3 ? L / H : 0), k3f = fwd3 ? L % H : 0;
     if (fwd3) {
 #pragma unroll
-      for (int i = 0; i < N; ++i) y[i] = __ldcg(S + (k3f * N + i) * N + k2f);
-      fft<float, N, -1>(y);
+      for (int i = 0; i < N; ++i) y[i] = from_c(__ldcg(S + (k3f * N + i) * N + k2f));
+      cfft<N, -1>(y);
     }
-    cl_arrive();
-    cl_wait();  // both CTAs hold their lines of the exchange buffer
+    cl_sync();  // both CTAs hold their lines of the exchange buffer
     if (fwd3) {
+      const float iv = 1.f / (float)V;
 #pragma unroll
-      for (int i = 0; i < N; ++i) __stcg(S + (k3f * N + i) * N + k2f, cscale(y[i], invV));
+      for (int i = 0; i < N; ++i) __stcg(S + (k3f * N + i) * N + k2f, to_c(vmul(y[i], vmk(iv, iv))));
     }
     if (tid < 6 * N) sPh[tid] = a.phase[tid];
-    // the gain spectrum of this CTA's k-slab starts at zero
-    for (int i = tid; i < N * MH * N; i += G::NT) sQG[i] = mk<C>(0.f, 0.f);
-    cl_arrive();
-    cl_wait();  // F and G complete in the scratch
+    cl_sync();  // F and G complete in the scratch
+    {
+      uint32_t t[2 * N];
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const C v = at(S, k1, lo, k);
+        tm_put(t, 2 * k, cre(v));
+        tm_put(t, 2 * k + 1, cim(v));
+      }
+      tm_store(tmF, t);
+      tmem_store_wait();
+    }
+    __syncthreads();
 
+    // Per direction two cluster barriers: #1 hands over the inverse
+    // transforms, #2 the forward one.  The h threads wait for #2 only after
+    // the first two passes of the next direction.
+    inverse12(0);
 #pragma unroll 1
     for (int pq = 0; pq < npq; ++pq) {
-      const int slot = pq & 1;
-      const C* ph = sPh + slot * 6 * N + fld * 3 * N;
-      // ---- pass 1: the field's line (k1, k2 = lo) along k3 -------------------
-      {
-        const int k1 = pair_kmap<N>(r, hi), k2 = lo;
-        const C e12 = cmul(ph[k1], ph[N + k2]);
-        const C* Sf = fld ? Gg : Fg;
-        C x[N];
-#pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = cmul(at(Sf, k1, k2, k), cmul(e12, ph[2 * N + k]));
-        fft<float, N, +1>(x);
-#pragma unroll
-        for (int k = 0; k < N; ++k) sW[(hi * N + k2) * LP + k] = x[k];
-      }
-      // the next (x, y)'s phases into the other slot
-      const C phn = (tid < 6 * N && pq + 1 < npq) ? a.phase[(size_t)(pq + 1) * 6 * N + tid] : mk<C>(0.f, 0.f);
-      __syncthreads();
-      if (tid < 6 * N && pq + 1 < npq) sPh[(slot ^ 1) * 6 * N + tid] = phn;
-      // ---- pass 2 and the exchange ------------------------------------------
-      const int xr = inverse_pass2();
+      const CM phn = (tid < 6 * N && pq + 1 < npq) ? a.phase[(size_t)(pq + 1) * 6 * N + tid] : make_float2(0.f, 0.f);
+      if (fld && pq > 0) cl_wait();  // #2 of the previous direction
+      cl_sync();                     // #1: both halves staged
       // ---- pass 3: g or h on the line (x2 = MH r + hi, x3 = lo) --------------
       C x[N];
-      pair_load3<float, N>(x, sW, xpeer(xr, fld), r, hi, lo);
-      fft<float, N, +1>(x);
-      __syncthreads();  // every thread has read its pass-3 inputs
+      load3(x, pq & 1);
+      cfft<N, 1>(x);
       if (fld) {
 #pragma unroll
-        for (int i = 0; i < N; ++i) sWh[(hi * N + lo) * LP + i] = x[i];
+        for (int i = 0; i < N; ++i) sH[i * NL] = x[i];
       }
-      __syncthreads();
+      if (tid < 6 * N && pq + 1 < npq) sPh[((pq + 1) & 1) * 6 * N + tid] = phn;
+      __syncthreads();  // h and the next phases in place
       // ---- g h, forward along x1; the k1 the peer owns go to its buffer ------
       if (!fld) {
 #pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = cmul(x[i], sWh[(hi * N + lo) * LP + i]);
-        fft<float, N, -1>(x);
-        C* const xs = xmine(xb, 0);
-        const int x2 = MH * r + hi;
-#pragma unroll
-        for (int k1 = 0; k1 < N; ++k1) {
-          if (pair_owner<N>(k1) == r) sWg[(pair_kinv<N>(k1) * N + x2) * LP + lo] = x[k1];
-          else __stcg(xs + (pair_kinv<N>(k1) * MH + hi) * N + lo, x[k1]);
+        for (int i = 0; i < N; ++i) {
+          const C h = sH[i * NL];
+          x[i] = vmk(cre(x[i]) * cre(h) - cim(x[i]) * cim(h), cre(x[i]) * cim(h) + cim(x[i]) * cre(h));
         }
-      }
-      cl_arrive();
-      cl_wait();  // both halves staged
-      const int xf = xb;
-      xb ^= 1;
-      // ---- forward along x2 on the lines (k1l, x3) ----------------------------
-      if (!fld) {
-        const C* xp = xpeer(xf, 0);
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-          x[j] = j / MH == r ? sWg[(hi * N + j) * LP + lo] : __ldcg(xp + (hi * MH + j % MH) * N + lo);
-        fft<float, N, -1>(x);
-#pragma unroll
-        for (int j = 0; j < N; ++j) sWg[(hi * N + j) * LP + lo] = x[j];
-      }
-      __syncthreads();
-      // ---- forward along x3 on the lines (k1l, k2); QGhat += b FFT(g h) ------
-      if (!fld) {
-        const int k1 = pair_kmap<N>(r, hi), k2 = lo;
-#pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = sWg[(hi * N + k2) * LP + k];
-        fft<float, N, -1>(x);
-        const C* bb = a.b + (size_t)pq * V + (k1 * N + k2) * N;
+        cfft<N, -1>(x);
+        CM* const xs = Xf + (r * 2 + (pq & 1)) * G::XSLAB + hi * N;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-          C* q = sQG + (k * MH + hi) * N + k2;
-          *q = cfma(__ldg(bb + k), x[k], *q);
+          if (pair_owner<N>(k) == r) w3p[pair_kinv<N>(k) * N * LP] = x[k];
+          else __stcg(xs + pair_kinv<N>(k) * MH * N, to_c(x[k]));
         }
       }
-      __syncthreads();
+      cl_arrive();  // #2
+      if (fld) {
+        if (pq + 1 < npq) inverse12(pq + 1);
+        continue;
+      }
+      cl_wait();
+      // ---- forward along x2 on the lines (k1l, x3) ----------------------------
+      const CM* const xp = Xf + ((r ^ 1) * 2 + (pq & 1)) * G::XSLAB + hi * MH * N;
+#pragma unroll
+      for (int j = 0; j < N; ++j) x[j] = j / MH == r ? w2p[j * LP] : from_c(__ldcg(xp + (j % MH) * N));
+      cfft<N, -1>(x);
+#pragma unroll
+      for (int j = 0; j < N; ++j) w2p[j * LP] = x[j];
+      group_sync();
+      // ---- forward along x3 on the lines (k1l, k2); QGhat += b FFT(g h) ------
+#pragma unroll
+      for (int k = 0; k < N; ++k) x[k] = w1p[k];
+      cfft<N, -1>(x);
+      const CM* bb = a.bt + (size_t)pq * V + k1 * N + lo;
+      tmem_store_wait();
+      sfor<0, N / 8>([&](auto cc) {
+        constexpr int c = decltype(cc)::value;
+        uint32_t t[16];
+        CM b[8];
+        tm_load(tmQ + 16 * c, t);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = __ldg(bb + (8 * c + i) * NN);
+        tm_wait(t);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const C v = x[8 * c + i];
+          const float q0 = pq == 0 ? 0.f : tm_get(t, 2 * i, 0.f), q1 = pq == 0 ? 0.f : tm_get(t, 2 * i + 1, 0.f);
+          tm_put(t, 2 * i, q0 + b[i].x * cre(v) - b[i].y * cim(v));
+          tm_put(t, 2 * i + 1, q1 + b[i].x * cim(v) + b[i].y * cre(v));
+        }
+        tm_store(tmQ + 16 * c, t);
+      });
+      if (pq + 1 < npq) inverse12(pq + 1);
     }
+    if (fld) cl_wait();  // #2 of the last direction
 
     // ---- QG = IFFT(QGhat) (field 0), fL = IFFT(c G) (field 1) ---------------
     {
-      const int k1 = pair_kmap<N>(r, hi), k2 = lo;
+      uint32_t t[2 * N];
+      tmem_store_wait();
+      tm_load(fld ? tmF : tmQ, t);
+      tm_wait(t);
       C x[N];
-      if (fld) {
-        const C* cc = a.c + (k1 * N + k2) * N;
 #pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = cmul(__ldg(cc + k), at(Gg, k1, k2, k));
-      } else {
-#pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = sQG[(k * MH + hi) * N + k2];
+      for (int k = 0; k < N; ++k) {
+        const float re = tm_get(t, 2 * k, 0.f), im = tm_get(t, 2 * k + 1, 0.f);
+        if (fld) {
+          const CM c = __ldg(a.c + (k1 * N + lo) * N + k);
+          x[k] = vmk(re * c.x - im * c.y, re * c.y + im * c.x);
+        } else {
+          x[k] = vmk(re, im);
+        }
       }
-      fft<float, N, +1>(x);
+      cfft<N, 1>(x);
 #pragma unroll
-      for (int k = 0; k < N; ++k) sW[(hi * N + k2) * LP + k] = x[k];
-    }
-    __syncthreads();
-    {
-      const int xr = inverse_pass2();
-      C x[N];
-      pair_load3<float, N>(x, sW, xpeer(xr, fld), r, hi, lo);
-      fft<float, N, +1>(x);
-      __syncthreads();
+      for (int k = 0; k < N; ++k) w1p[k] = x[k];
+      pass2_out(npq & 1);
+      cl_sync();
+      load3(x, npq & 1);
+      cfft<N, 1>(x);
       if (fld) {
 #pragma unroll
-        for (int i = 0; i < N; ++i) sWh[(hi * N + lo) * LP + i] = x[i];
+        for (int i = 0; i < N; ++i) sH[i * NL] = x[i];
       }
       __syncthreads();
       if (!fld) {
         // x2 = MH r + hi, x3 = lo: bank entries v = x1 N^2 + x2 N + x3
-        const int64_t b0 = soa_ix(upt, a.ldim, elem, (int64_t)(MH * r + hi) * N + lo, V, a.soasz);
+        const int64_t b0 = soa_ix(upt, a.ldim, elem, (int64_t)x2 * N + lo, V, a.soasz);
         const int64_t st = (int64_t)NN * a.soasz;
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-          const float qv = a.prefac * (x[i].x - a.fp[b0 + i * st] * sWh[(hi * N + lo) * LP + i].x);
+          const float qv = a.prefac * (cre(x[i]) - a.fp[b0 + i * st] * cre(sH[i * NL]));
           a.Q[b0 + i * st] = a.accumulate ? a.Q[b0 + i * st] + qv : qv;
         }
       }
     }
     // the next point rewrites the scratch and the work cubes: both CTAs done
-    cl_arrive();
-    cl_wait();
+    cl_sync();
   }
-  cl_arrive();
-  cl_wait();  // no CTA leaves while the peer may still address its memory
+  if (tid < 32) tmem_dealloc(s_tmem, G::TCOLS);
+  cl_sync();  // no CTA leaves while the peer may still address its memory
 }
 
 }  // namespace dgfs

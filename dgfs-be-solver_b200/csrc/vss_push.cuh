@@ -41,6 +41,7 @@ template <typename T> struct VssArgs {
   int P, M;
   const cx<T>* phase;  // [P][M][2][3][N]: field 0 e^{+i kq fac s[ax] l0}, field 1 e^{-i kp fac s[ax] l0}
   const cx<T>* b;      // [P][M][V] w_x b_xy
+  const cx<T>* bt;     // [P][M][N][N*N] the same, last axis outermost (two-CTA kernel)
   const cx<T>* c;      // [V] loss kernel
   cx<T>* fc;           // scratch [gridDim.x][N][NJ]: gain spectrum per CTA
   int* err;
