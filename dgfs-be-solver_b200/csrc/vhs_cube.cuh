@@ -102,18 +102,26 @@ template <typename T, int N> struct CubeGeom {
 // Radial-node chunks per point.  A launch with few points would leave SMs
 // idle with one point per CTA, so each point's P radial nodes can be split
 // into P work items of one node each: cost ~ waves x (nodes per item x
-// (3 M + 3) + 3) passes (the 3: every item transforms f itself).  Only 1 or
+// (3 M + 3) + kFixed) passes.  kFixed is what an item costs before its first
+// node and after its last (its own transform of f, the tables, the slice and
+// the point's last pass), fitted from the time per wave of split and of whole
+// items: 59 passes at N = 24 (P = 12, M = 16: 172 against 1,048 us a wave),
+// 48 at N = 16 FP32 (P = 8, M = 6: 38 against 117 us) and 43 in FP64 (56
+// against 185 us).  So a split pays up to 6, 3 and 3 waves: 74 points at
+// N = 24 take 1,048 us split and 1,062 us whole, 98 points 1,390 against 1,062 us;
+// 49 at N = 16 take 125 against 131 us (FP64 182 against 201 us), 61 points
+// 163 against 131 us (239 against 201 us).  Only 1 or
 // P chunks: with one node per chunk the final sum over the chunks' slices
 // adds the nodes in the same order as the unsplit accumulation, so a point's
 // Q does not depend on the launch it is part of (bit for bit).  Items are
-// capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch:
-// with P = 12 a split covers up to two waves of whole points).  Every CTA
-// computes the same value.
+// capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch).
+// Every CTA computes the same value.
 __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
   if (P < 2 || (long long)npts * P > (long long)kCubeSlices * G) return 1;
+  constexpr double kFixed = 48.0;
   const double per_node = 3.0 * M + 3.0;
-  const double whole = (double)((npts + G - 1) / G) * (P * per_node + 3.0);
-  const double split = (double)(((long long)npts * P + G - 1) / G) * (per_node + 3.0);
+  const double whole = (double)((npts + G - 1) / G) * (P * per_node + kFixed);
+  const double split = (double)(((long long)npts * P + G - 1) / G) * (per_node + kFixed);
   return split < whole ? P : 1;
 }
 

@@ -56,3 +56,25 @@ def test_line_kernels_across_splits(name, precision, kw, project, neles):
         sm.fs(fin, one, neles - 1, 0)
         np.testing.assert_array_equal(one.get()[0, :, neles - 1],
                                       Q[:, neles - 1])
+
+
+@pytest.mark.parametrize('precision,Nv,P,M', [
+    ('single', 16, 8, 6), ('single', 24, 12, 16), ('double', 16, 8, 6)])
+def test_split_rule_does_not_change_values(precision, Nv, P, M):
+    """Banks on both sides of each wave of split and whole items: every
+    point equals the value it has in a launch of its own."""
+    cfg = config('channel-n32', precision, Nv=Nv, Nrho=P, M=M)
+    be, vm, sm = _model(cfg)
+    neles = 150
+    base = random_states(vm.cv(), 3, seed=Nv)
+    fin, ref = _bank(be, vm, base[np.arange(neles) % 3][None])
+    for pt in range(3):
+        sm.fs_range(fin, ref, pt, 1)
+    want = ref.get()[0, :, :3]
+    for n in (18, 37, 49, 55, 56, 74, 75, 90, 91, 147, 148, 149):
+        _, out = _bank(be, vm, base[np.arange(neles) % 3][None])
+        sm.fs_range(fin, out, 0, n)
+        sm.status()
+        got = out.get()[0]
+        for e in range(n):
+            np.testing.assert_array_equal(got[:, e], want[:, e % 3])
