@@ -242,6 +242,7 @@ class MLP:
         self.err = torch.zeros(1, dtype=torch.int32, device=device)
         self.sync_bf16()
         self._cache = None
+        self._sides = []
 
     @property
     def _s(self):
@@ -286,6 +287,21 @@ class MLP:
                                  'a bounded wait of the tensor-core GEMM '
                                  'ran out')
 
+    def _fork(self, i):
+        """Side stream i of this network, behind the current stream: work
+        whose results the current stream needs only at the next join runs
+        beside it (as parallel branches when captured in a CUDA graph)."""
+        cur = torch.cuda.current_stream(self.device)
+        while len(self._sides) <= i:
+            self._sides.append(torch.cuda.Stream(device=self.device))
+        self._sides[i].wait_stream(cur)
+        return torch.cuda.stream(self._sides[i])
+
+    def _join(self, *sides):
+        cur = torch.cuda.current_stream(self.device)
+        for i in sides:
+            cur.wait_stream(self._sides[i])
+
     def _gemm_bf16(self, A, a_mn, lda, B, b_mn, ldb, C, M, N, K, bias=None,
                    act=0, acc=0, Cb=None):
         _lib.check(_lib.load().dgfs_mlp_gemm_bf16(
@@ -311,16 +327,18 @@ class MLP:
               for i in (1, 2, 3)]
         Y = ws.get('trainY', (B, nout))
         self._to_bf16(X, Xb)
+        # the linear skip beside the layers; the last product adds to it
+        with self._fork(0):
+            self._gemm_bf16(Xb, 0, nin, wb['Ws'], 1, nout, Y, B, nout, nin)
         self._gemm_bf16(Xb, 0, nin, wb['W1'], 1, wd, H[0], B, wd, nin,
                         w['b1'], act=1, Cb=Hb[0])
         self._gemm_bf16(Hb[0], 0, wd, wb['W2'], 1, wd, H[1], B, wd, wd,
                         w['b2'], act=1, Cb=Hb[1])
         self._gemm_bf16(Hb[1], 0, wd, wb['W3'], 1, wd, H[2], B, wd, wd,
                         w['b3'], act=1, Cb=Hb[2])
+        self._join(0)
         self._gemm_bf16(Hb[2], 0, wd, wb['W4'], 1, nout, Y, B, nout, wd,
-                        w['b4'])
-        self._gemm_bf16(Xb, 0, nin, wb['Ws'], 1, nout, Y, B, nout, nin,
-                        acc=1)
+                        w['b4'], acc=1)
         self._cache = (X, H[0], H[1], H[2])
         self._cache_bf16 = (Xb, Hb[0], Hb[1], Hb[2])
         return Y
@@ -337,35 +355,39 @@ class MLP:
         g, wb, ws = self.g, self.wb, self.ws
         dYb = ws.get('dYb', (B, nout), torch.bfloat16)
         dH = ws.get('dH', (B, wd))
-        dZ = ws.get('dZ', (B, wd))
-        dZb = ws.get('dZb', (B, wd), torch.bfloat16)
         self._to_bf16(dY, dYb)
 
-        def wgrad(Ab, Db, name, k, n):
-            self._gemm_bf16(Ab, 1, k, Db, 1, n, g[name], k, n, B)
+        def grads(A, D, Db, wname, bname, k, n):
+            """Weight and bias gradients of a layer, beside the chain of
+            input gradients (their own streams)."""
+            with self._fork(0):
+                self._gemm_bf16(A, 1, k, Db, 1, n, g[wname], k, n, B)
+            if bname is not None:
+                with self._fork(1):
+                    _lib.check(lib.dgfs_mlp_colsum(
+                        B, n, _p(D), n, _p(g[bname]), 0, self._s),
+                        'dgfs_mlp_colsum')
 
-        def bgrad(D, name, n):
-            _lib.check(lib.dgfs_mlp_colsum(B, n, _p(D), n, _p(g[name]), 0,
-                                           self._s), 'dgfs_mlp_colsum')
-
-        def through(Db, nd, W, H):
+        def through(Db, nd, W, H, i):
+            # each layer's dZ has buffers of its own: the gradient products
+            # on the side streams still read it while the chain goes on
+            dZ = ws.get('dZ%d' % i, (B, wd))
+            dZb = ws.get('dZ%db' % i, (B, wd), torch.bfloat16)
             self._gemm_bf16(Db, 0, nd, W, 0, nd, dH, B, wd, nd)
             _lib.check(lib.dgfs_mlp_tanh_bwd_bf16(
                 dH.numel(), _p(H), _p(dH), _p(dZ), _p(dZb), self._s),
                 'dgfs_mlp_tanh_bwd_bf16')
+            return dZ, dZb
 
-        wgrad(H3b, dYb, 'W4', wd, nout)
-        bgrad(dY, 'b4', nout)
-        wgrad(Xb, dYb, 'Ws', nin, nout)
-        through(dYb, nout, wb['W4'], H3)
-        wgrad(H2b, dZb, 'W3', wd, wd)
-        bgrad(dZ, 'b3', wd)
-        through(dZb, wd, wb['W3'], H2)
-        wgrad(H1b, dZb, 'W2', wd, wd)
-        bgrad(dZ, 'b2', wd)
-        through(dZb, wd, wb['W2'], H1)
-        wgrad(Xb, dZb, 'W1', nin, wd)
-        bgrad(dZ, 'b1', wd)
+        grads(H3b, dY, dYb, 'W4', 'b4', wd, nout)
+        grads(Xb, dY, dYb, 'Ws', None, nin, nout)
+        dZ, dZb = through(dYb, nout, wb['W4'], H3, 3)
+        grads(H2b, dZ, dZb, 'W3', 'b3', wd, wd)
+        dZ, dZb = through(dZb, wd, wb['W3'], H2, 2)
+        grads(H1b, dZ, dZb, 'W2', 'b2', wd, wd)
+        dZ, dZb = through(dZb, wd, wb['W2'], H1, 1)
+        grads(Xb, dZ, dZb, 'W1', 'b1', nin, wd)
+        self._join(0, 1)
         return g
 
     def forward(self, X, keep=False, mcount=None):
@@ -734,6 +756,7 @@ class VHSSurrogate:
         main = torch.cuda.current_stream(self.device)
         if self._side is None:
             self._side = torch.cuda.Stream(device=self.device)
+            self._side_nu = torch.cuda.Stream(device=self.device)
             self._fork = torch.cuda.Event()
             self._join = torch.cuda.Event()
         self._fork.record(main)
@@ -743,10 +766,14 @@ class VHSSurrogate:
             neles, ldim, self.backend.soasz, _p(plain), _p(nplain), npts,
             self._side.cuda_stream), 'dgfs_vhs_apply_list')
         self._join.record(self._side)
-        nu = self.loss_rate(fbank, self.nu_bank(fbank), gate)
-        # the network runs on the gate-1 rows only
+        # the collision frequency and the network (on the gate-1 rows only)
+        # both need nothing but the gate: side by side
+        self._side_nu.wait_event(self._fork)
+        with torch.cuda.stream(self._side_nu):
+            nu = self.loss_rate(fbank, self.nu_bank(fbank), gate)
         Bp = self.scale_targets(self.predict(X, net, nnet), eps,
                                 inverse=True)
+        main.wait_stream(self._side_nu)
         work = ws.get('rwork', (nupts*(-(-neles//32))*32*(32*5 + NMODES),),
                       torch.float64)
         _lib.check(lib.dgfs_hermite_reconstruct(
