@@ -189,3 +189,30 @@ def test_tma_gemm_accumulates():
     C0 = torch.randn(M, N, generator=g).to(DEV)
     C, _, _ = _run_bf16(M, N, K, X, 1, M, D, 1, N, acc=1, C0=C0)
     _check(C, C0.double() + X.double().T @ D.double())
+
+
+@pytest.mark.parametrize('M,N', [(1, 8), (7, 64), (8, 56), (9, 33), (31, 129),
+                                 (33, 128), (127, 40), (129, 72)])
+def test_tma_gemm_accumulates_at_ragged_tiles(M, N):
+    """Accumulation where the last group of rows, the last warp's rows and
+    the last columns of a tile are partly outside C; with bias, tanh and the
+    pre-activation; nothing outside M x N is written."""
+    K = 64
+    g = torch.Generator(device='cpu').manual_seed(M + 1000*N)
+    A = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    B = (torch.randn(N, K, generator=g)/8).to(torch.bfloat16).to(DEV)
+    b = (0.1*torch.randn(N, generator=g)).to(DEV)
+    C0 = torch.full((M + 2, N), 7.0, device=DEV)
+    C0[:M] = torch.randn(M, N, generator=g).to(DEV)
+    C, Z, Cb = C0.clone(), torch.full_like(C0, 7.0), None
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _lib.check(_lib.load().dgfs_mlp_gemm_bf16(
+        M, N, K, A.data_ptr(), 0, K, B.data_ptr(), 0, K, b.data_ptr(),
+        Z.data_ptr(), C.data_ptr(), None, N, 1, 1, err.data_ptr(),
+        torch.cuda.current_stream().cuda_stream), 'dgfs_mlp_gemm_bf16')
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    z = A.double() @ B.double().T + b.double() + C0[:M].double()
+    _check(Z[:M], z)
+    _check(C[:M], torch.tanh(z))
+    assert torch.all(C[M:] == 7.0) and torch.all(Z[M:] == 7.0)
