@@ -32,22 +32,20 @@ __device__ __forceinline__ float ld_b(const __nv_bfloat16* p) { return __bfloat1
 // C[m][n] (ldc) = act(sum_k A(m,k) B(k,n) + bias[n]) (+ C if accumulate);
 // BM x BN tile per CTA, TM x TN outputs per thread (256 threads), BK-deep
 // slices of K staged in shared memory (deeper slices for small tiles: fewer
-// round trips to L2 per output).  With mcount, only the first *mcount rows
-// exist (a count the device produced): tiles past it return at once.
+// round trips to L2 per output).
+template <int BM, int BN, int BK> constexpr int kTileFloats = BK * (BM + 4) + BK * (BN + 4);
 template <typename TB, int BM, int BN, int TM, int TN, int BK>
-__global__ void __launch_bounds__(NTH) gemm_kernel(int M, const int* __restrict__ mcount, int N, int K,
-                                                  const float* __restrict__ A, long long sam, long long sak,
-                                                  const TB* __restrict__ B, long long sbk, long long sbn,
-                                                  const float* __restrict__ bias, float* __restrict__ Z,
-                                                  float* __restrict__ C, long long ldc, int act, int accumulate) {
+__device__ __forceinline__ void gemm_tile(float* smem, int M, int N, int K, const float* __restrict__ A,
+                                          long long sam, long long sak, const TB* __restrict__ B, long long sbk,
+                                          long long sbn, const float* __restrict__ bias, float* __restrict__ Z,
+                                          float* __restrict__ C, long long ldc, int act, int accumulate) {
   static_assert((BM / TM) * (BN / TN) == NTH, "one output block per thread");
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
+  float(*const As)[BM + 4] = reinterpret_cast<float(*)[BM + 4]>(smem);
+  float(*const Bs)[BN + 4] = reinterpret_cast<float(*)[BN + 4]>(smem + BK * (BM + 4));
   constexpr int TX = BN / TN;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  if (mcount) M = min(M, *mcount);
-  if (m0 >= M) return;  // uniform over the CTA
+  if (m0 >= M || n0 >= N) return;  // uniform over the CTA
   float acc[TM][TN] = {};
   // slices of K go through registers: every global load of a slice is
   // issued before any of its shared-memory stores, and the next slice's
@@ -117,6 +115,114 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(int M, const int* __restrict_
       C[m * ldc + n] = act == 1 ? tanhf(z) : z;
     }
   }
+}
+
+template <typename TB, int BM, int BN, int TM, int TN, int BK>
+__global__ void __launch_bounds__(NTH, 2) gemm_kernel(int M, int N, int K, const float* __restrict__ A, long long sam,
+                                                  long long sak, const TB* __restrict__ B, long long sbk,
+                                                  long long sbn, const float* __restrict__ bias,
+                                                  float* __restrict__ Z, float* __restrict__ C, long long ldc,
+                                                  int act, int accumulate) {
+  __shared__ __align__(16) float smem[kTileFloats<BM, BN, BK>];
+  gemm_tile<TB, BM, BN, TM, TN, BK>(smem, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate);
+}
+
+// The same product, bit for bit (each sum runs over k in ascending order), for
+// few rows: 32 x 8 tiles, one output per thread, 256-deep slices.  Few rows are
+// few CTAs, each a chain of slices of K behind one another: with 32 x 32 tiles
+// and 64-deep slices one product of 32 x 512 x 512 took 16 us.  Here K = 512 is
+// two trips to L2 and four times as many SMs share the columns: 9.4 us (1 to 64 rows;
+// for 96 rows, two waves, 16.1 against 16.1 us, for 256 rows 30.8 against
+// 16.3 us).  So it is taken while its tiles are one wave and K is more than half
+// a slice (K = 24, zero-filled: 5.0 against 3.8 us), on
+// the device where only the device knows the row count: above, the CTAs take
+// the 32 x 32 tiles.  With mcount, only the first *mcount rows exist: tiles past
+// it return at once.
+constexpr int FRM = 32, FRN = 8, FRK = 256, FRS = FRK + 4;  // FRS: lanes 4 banks apart
+constexpr int kRowsTiles = 148;
+static_assert(FRM * FRN == NTH, "one output per thread");
+
+template <typename TB>
+__global__ void __launch_bounds__(NTH) gemm_rows_kernel(int M, const int* __restrict__ mcount, int N, int K,
+                                                        const float* __restrict__ A, long long sam, long long sak,
+                                                        const TB* __restrict__ B, long long sbk, long long sbn,
+                                                        const float* __restrict__ bias, float* __restrict__ Z,
+                                                        float* __restrict__ C, long long ldc, int act,
+                                                        int accumulate, int max_tiles) {
+  __shared__ __align__(16) float smem[(FRM + FRN) * FRS];
+  static_assert(kTileFloats<32, 32, 64> <= (FRM + FRN) * FRS, "shared memory of both forms");
+  float* const As = smem;              // [m][k]
+  float* const Bs = smem + FRM * FRS;  // [n][k]
+  const int m0 = blockIdx.y * FRM, n0 = blockIdx.x * FRN;
+  if (mcount) M = min(M, *mcount);
+  if ((long long)((M + FRM - 1) / FRM) * gridDim.x > max_tiles) {  // the grid covers these tiles too
+    gemm_tile<TB, 32, 32, 2, 2, 64>(smem, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate);
+    return;
+  }
+  if (m0 >= M) return;  // uniform over the CTA
+  constexpr int LA = FRM * FRK / NTH, LB = FRN * FRK / NTH;
+  float ra[LA], rb[LB];
+  // consecutive threads walk k when A is row-major (sak == 1), m otherwise; n
+  // when B is row-major, k otherwise
+  auto a_ix = [&](int u, int& mm, int& kk) {
+    const int t = threadIdx.x + u * NTH;
+    mm = sak == 1 ? t / FRK : t % FRM;
+    kk = sak == 1 ? t % FRK : t / FRM;
+  };
+  auto b_ix = [&](int u, int& nn, int& kk) {
+    const int t = threadIdx.x + u * NTH;
+    nn = sbn == 1 ? t % FRN : t / FRK;
+    kk = sbn == 1 ? t / FRN : t % FRK;
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < LA; ++u) {
+      int mm, kk;
+      a_ix(u, mm, kk);
+      ra[u] = (m0 + mm < M && k0 + kk < K) ? A[(m0 + mm) * sam + (k0 + kk) * sak] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      int nn, kk;
+      b_ix(u, nn, kk);
+      rb[u] = (n0 + nn < N && k0 + kk < K) ? ld_b(B + (k0 + kk) * sbk + (n0 + nn) * sbn) : 0.f;
+    }
+  };
+  const int n = n0 + threadIdx.x % FRN, m = m0 + threadIdx.x / FRN;
+  const float* const ap = As + threadIdx.x / FRN * FRS;
+  const float* const bp = Bs + threadIdx.x % FRN * FRS;
+  float acc = 0.f;
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += FRK) {
+#pragma unroll
+    for (int u = 0; u < LA; ++u) {
+      int mm, kk;
+      a_ix(u, mm, kk);
+      As[mm * FRS + kk] = ra[u];
+    }
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      int nn, kk;
+      b_ix(u, nn, kk);
+      Bs[nn * FRS + kk] = rb[u];
+    }
+    __syncthreads();
+    if (k0 + FRK < K) fetch(k0 + FRK);
+#pragma unroll 8
+    for (int kk = 0; kk < FRK; kk += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(ap + kk), b = *reinterpret_cast<const float4*>(bp + kk);
+      acc = fmaf(a.x, b.x, acc);
+      acc = fmaf(a.y, b.y, acc);
+      acc = fmaf(a.z, b.z, acc);
+      acc = fmaf(a.w, b.w, acc);
+    }
+    __syncthreads();
+  }
+  if (m >= M || n >= N) return;
+  float z = acc + (bias ? bias[n] : 0.f);
+  if (accumulate) z += C[m * ldc + n];
+  if (Z) Z[m * ldc + n] = z;
+  C[m * ldc + n] = act == 1 ? tanhf(z) : z;
 }
 
 __global__ void tanh_bwd_kernel(long long n, const float* __restrict__ H, const float* __restrict__ dH,
@@ -268,25 +374,32 @@ inline int launched(const char* what) {
 }  // namespace
 
 template <typename TB, int BM, int BN, int TM, int TN, int BK>
-static void gemm_launch(int M, const int* mcount, int N, int K, const float* A, long long sam, long long sak,
-                        const TB* B, long long sbk, long long sbn, const float* bias, float* Z, float* C,
-                        long long ldc, int act, int accumulate, cudaStream_t s) {
+static void gemm_launch(int M, int N, int K, const float* A, long long sam, long long sak, const TB* B,
+                        long long sbk, long long sbn, const float* bias, float* Z, float* C, long long ldc, int act,
+                        int accumulate, cudaStream_t s) {
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  gemm_kernel<TB, BM, BN, TM, TN, BK><<<grid, NTH, 0, s>>>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc,
-                                                       act, accumulate);
+  gemm_kernel<TB, BM, BN, TM, TN, BK><<<grid, NTH, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act,
+                                                           accumulate);
 }
 
 template <typename TB>
-static void gemm_pick(int M, const int* mcount, int N, int K, const float* A, long long sam, long long sak,
-                      const TB* B, long long sbk, long long sbn, const float* bias, float* Z, float* C,
-                      long long ldc, int act, int accumulate, cudaStream_t s) {
-  // 64 x 64 tiles when they fill the GPU; 32 x 32 for short products and
-  // for row counts known only on the device (typically a few dozen rows)
+static int gemm_pick(int M, const int* mcount, int N, int K, const float* A, long long sam, long long sak,
+                     const TB* B, long long sbk, long long sbn, const float* bias, float* Z, float* C,
+                     long long ldc, int act, int accumulate, cudaStream_t s) {
+  // 64 x 64 tiles when they fill the GPU; 32 x 8 tiles for few rows (see
+  // gemm_rows_kernel, which also takes the row counts only the device knows);
+  // 32 x 32 tiles between.  The three give the same bits
   const long long tiles64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  const dim3 fr((N + FRN - 1) / FRN, (M + FRM - 1) / FRM);
+  const int max_tiles = K > FRK / 2 ? kRowsTiles : 0;
   if (!mcount && tiles64 >= 148)
-    gemm_launch<TB, 64, 64, 4, 4, 16>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
+    gemm_launch<TB, 64, 64, 4, 4, 16>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
+  else if (mcount || (long long)fr.x * fr.y <= max_tiles)
+    gemm_rows_kernel<TB><<<fr, NTH, 0, s>>>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act,
+                                            accumulate, max_tiles);
   else
-    gemm_launch<TB, 32, 32, 2, 2, 64>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
+    gemm_launch<TB, 32, 32, 2, 2, 64>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
+  return launched("gemm");
 }
 
 extern "C" int dgfs_mlp_gemm(int M, int N, int K, const float* A, long long sam, long long sak, const void* B,
@@ -297,12 +410,10 @@ extern "C" int dgfs_mlp_gemm(int M, int N, int K, const float* A, long long sam,
   if (act != 0 && act != 1) return dgfs::set_error(DGFS_ERR_INVALID, "act must be 0 or 1");
   if ((M + 31) / 32 > 65535) return dgfs::set_error(DGFS_ERR_UNSUPPORTED, "M=%d too large", M);
   if (b_bf16)
-    gemm_pick<__nv_bfloat16>(M, mcount, N, K, A, sam, sak, (const __nv_bfloat16*)B, sbk, sbn, bias, Z, C, ldc,
-                             act, accumulate, (cudaStream_t)stream);
-  else
-    gemm_pick<float>(M, mcount, N, K, A, sam, sak, (const float*)B, sbk, sbn, bias, Z, C, ldc, act, accumulate,
-                     (cudaStream_t)stream);
-  return launched("gemm");
+    return gemm_pick<__nv_bfloat16>(M, mcount, N, K, A, sam, sak, (const __nv_bfloat16*)B, sbk, sbn, bias, Z, C, ldc,
+                                    act, accumulate, (cudaStream_t)stream);
+  return gemm_pick<float>(M, mcount, N, K, A, sam, sak, (const float*)B, sbk, sbn, bias, Z, C, ldc, act, accumulate,
+                          (cudaStream_t)stream);
 }
 
 extern "C" int dgfs_mlp_tanh_bwd(long long n, const float* H, const float* dH, float* dZ, void* stream) {

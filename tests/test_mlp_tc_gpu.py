@@ -216,3 +216,43 @@ def test_tma_gemm_accumulates_at_ragged_tiles(M, N):
     _check(Z[:M], z)
     _check(C[:M], torch.tanh(z))
     assert torch.all(C[M:] == 7.0) and torch.all(Z[M:] == 7.0)
+
+
+@pytest.mark.parametrize('M,N,K', [(1, 512, 512), (33, 9, 129), (64, 512, 257),
+                                   (65, 512, 256), (96, 40, 128),
+                                   (300, 512, 512)])
+@pytest.mark.parametrize('lay', [0, 1])
+def test_simt_tile_forms_agree(M, N, K, lay):
+    """The SIMT product's tile forms give the same bits: a device row count
+    (few rows: 32 x 8 tiles; many: 32 x 32) against the same rows of a
+    product large enough for 64 x 64 tiles, in both operand layouts; rows
+    past the count are left alone.  Against the FP64 product, K FP32
+    roundings of a sum of terms of order 1: K 2^-24 of the largest sum of
+    magnitudes, below 1e-4 here."""
+    g = torch.Generator(device='cpu').manual_seed(M + 7*N + K)
+    big = max(M, 64*148*64//max(N, 64) + 64)
+    A = torch.randn(big, K, generator=g).to(DEV)
+    B = torch.randn(K, N, generator=g).to(torch.bfloat16).to(DEV)
+    b = torch.randn(N, generator=g).to(DEV)
+    At, Bt = (A.T.contiguous(), B.T.contiguous()) if lay else (A, B)
+    lib = _lib.load()
+
+    def run(rows, count):
+        C = torch.full((rows, N), 7.0, device=DEV)
+        _lib.check(lib.dgfs_mlp_gemm(
+            rows, N, K, At.data_ptr(), 1 if lay else K, big if lay else 1,
+            Bt.data_ptr(), 1, 1 if lay else N, K if lay else 1, b.data_ptr(),
+            None, C.data_ptr(), N, 0, 0,
+            None if count is None else count.data_ptr(),
+            torch.cuda.current_stream().cuda_stream), 'dgfs_mlp_gemm')
+        torch.cuda.synchronize()
+        return C
+
+    full = run(big, None)
+    ref = A[:M].double() @ B.double() + b.double()
+    assert float((full[:M].double() - ref).abs().max()) < \
+        1e-4*max(1.0, float(ref.abs().max()))
+    assert torch.equal(run(M, None), full[:M])
+    cnt = torch.tensor([M], dtype=torch.int32, device=DEV)
+    part = run(M + 40, cnt)
+    assert torch.equal(part[:M], full[:M]) and torch.all(part[M:] == 7.0)
