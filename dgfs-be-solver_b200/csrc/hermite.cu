@@ -29,7 +29,9 @@
 //               energy moments.
 // The velocity grid is a tensor product, so every sum factorises into three
 // 1D contractions.  One CTA per solution point.
+#include <algorithm>
 #include <cmath>
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
 #include "../../include/dgfs_b200.h"
@@ -68,37 +70,34 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   double s = 0;
-  for (int w = 0; w < kThreads / 32; ++w) s += red[w];
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) s += red[w];
   return s;
 }
 
 // rho, u, T of the point's distribution (one pass, FP64):
 // T = (2/3) (sum f |c|^2 / sum f - |u|^2); the cancellation costs
 // |u|^2/T ulps, far below the FP32 bank's own rounding
-template <typename T>
-__device__ void point_frame(const T* f, int upt, int e, const FrameArgs& a, double* red, double* mom) {
+// A thread takes the row (I, J) = r; val(K) is the row's value at K.
+template <typename Val>
+__device__ __forceinline__ void point_frame(const Val& val, int r, const FrameArgs& a, double* red, double* mom) {
   const int N = a.N;
-  const long long V = (long long)N * N * N;
   const double h = 2.0 * a.L / N, c00 = -a.L + a.L / N;
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-  const long long b0 = dgfs::soa_ix(upt, a.ldim, e, 0, V, 32);
-  // rows (I, J) along K, as project_modes reads them
-  for (int r = threadIdx.x; r < N * N; r += kThreads) {
+  if (r < N * N) {
     const double cx = c00 + (r / N) * h, cy = c00 + (r % N) * h;
-    double t0 = 0, tz = 0, tzz = 0;
+    double tz = 0, tzz = 0;
 #pragma unroll 4
     for (int K = 0; K < N; ++K) {
-      const double fv = (double)f[b0 + ((long long)r * N + K) * 32];
+      const double fv = val(K);
       const double cz = c00 + K * h;
-      t0 += fv;
+      s0 += fv;
       tz += fv * cz;
       tzz += fv * cz * cz;
     }
-    s0 += t0;
-    s1 += t0 * cx;
-    s2 += t0 * cy;
-    s3 += tz;
-    s4 += t0 * (cx * cx + cy * cy) + tzz;
+    s1 = s0 * cx;
+    s2 = s0 * cy;
+    s3 = tz;
+    s4 = s0 * (cx * cx + cy * cy) + tzz;
   }
   const double m0 = block_sum(s0, red), m1 = block_sum(s1, red), m2 = block_sum(s2, red),
                m3 = block_sum(s3, red), m4 = block_sum(s4, red);
@@ -135,71 +134,59 @@ __device__ void basis_tables(const FrameArgs& a, const double* mom, double (*H)[
   }
 }
 
-// Fields projected by project_modes: a bank value, or the gain deviation
-// G - nu M = Q + nu (f - M) of a collision bank Q given the collision
-// frequency nu and the local Maxwellian M (value Mv at the node).
-template <typename T> struct BankField {
-  const T* g;
-  __device__ double operator()(long long ix, double) const { return (double)g[ix]; }
-};
-template <typename T> struct DevField {  // f - M
-  const T* f;
-  __device__ double operator()(long long ix, double Mv) const { return (double)f[ix] - Mv; }
-};
-template <typename T> struct GainDevField {
-  const T *q, *nu, *f;
-  __device__ double operator()(long long ix, double Mv) const {
-    return (double)q[ix] + (double)nu[ix] * ((double)f[ix] - Mv);
-  }
-};
-
-// out[m] = cw sum_v chi g(c_v) phi_m(c^_v) for the 220 modes
+// out[m] = cw sum_v chi g(c_v) phi_m(c^_v) for the 220 modes; one thread per
+// row (I, J) = r of the velocity grid, g(K, Mv) the row's field at K given
+// the local Maxwellian Mv there.  t1 may share its memory with what g reads.
 // The window chi is evaluated in FP32 (erfcf): it only shapes the
 // projection, and the coefficients leave in FP32.
 template <typename Field>
-__device__ void project_modes(const Field& g, int upt, int e, const FrameArgs& a, const double* mom,
-                              double (*H)[kMaxN][kP], double (*Ex)[kMaxN], double* t1, double* t2,
-                              double* out) {
-  const int N = a.N;
-  const long long V = (long long)N * N * N;
+__device__ __forceinline__ void project_modes(const Field& g, int r, const FrameArgs& a, const double* mom,
+                                              double (*H)[kMaxN][kP], double (*Ex)[kMaxN], double* t1, double* t2,
+                                              double* out) {
+  const int N = a.N, PS = N * N + 1;  // t1 [k][r], planes one entry apart in the banks
   const double h = 2.0 * a.L / N, c00 = -a.L + a.L / N, rt = rsqrt(mom[4]);
   // local Maxwellian rho T^{-3/2} pi^{-3/2} e^{-|c^|^2}
   const double m0 = mom[0] * rt * rt * rt * 0.17958712212516656;
-  // t1[I][J][k] = sum_K chi g[I][J][K] Hz[K][k]
-  for (int r = threadIdx.x; r < N * N; r += kThreads) {
-    double acc[kP];
+  // t1[k][I][J] = sum_K chi g[I][J][K] Hz[K][k]
+  double acc[kP];
 #pragma unroll
-    for (int k = 0; k < kP; ++k) acc[k] = 0;
+  for (int k = 0; k < kP; ++k) acc[k] = 0;
+  if (r < N * N) {
     const int I = r / N, J = r % N;
     const double dx = (c00 + I * h - mom[1]) * rt, dy = (c00 + J * h - mom[2]) * rt;
     const double r2xy = dx * dx + dy * dy, mxy = m0 * Ex[0][I] * Ex[1][J];
-    const long long b0 = dgfs::soa_ix(upt, a.ldim, e, (long long)r * N, V, 32);
     for (int K = 0; K < N; ++K) {
       const double dz = (c00 + K * h - mom[3]) * rt;
       const float r2 = (float)(r2xy + dz * dz);
       const double chi = 0.5f * erfcf((sqrtf(r2) - (float)kWinR) * (float)(1.0 / kWinW));
-      const double gv = chi * g(b0 + (long long)K * 32, mxy * Ex[2][K]);
+      const double gv = chi * g(K, mxy * Ex[2][K]);
 #pragma unroll
       for (int k = 0; k < kP; ++k) acc[k] += gv * H[2][K][k];
     }
+  }
+  __syncthreads();
+  if (r < N * N) {
 #pragma unroll
-    for (int k = 0; k < kP; ++k) t1[r * kP + k] = acc[k];
+    for (int k = 0; k < kP; ++k) t1[k * PS + r] = acc[k];
   }
   __syncthreads();
-  // t2[I][j][k] = sum_J t1[I][J][k] Hy[J][j]   (j + k <= 9)
-  for (int t = threadIdx.x; t < N * kP * kP; t += kThreads) {
-    const int I = t / (kP * kP), j = (t / kP) % kP, k = t % kP;
+  // t2[I][k][j] = sum_J t1[k][I][J] Hy[J][j]   (j + k <= 9)
+  for (int t = threadIdx.x; t < N * kP * kP; t += blockDim.x) {
+    const int I = t / (kP * kP), k = (t / kP) % kP, j = t % kP;
     if (j + k > kDeg) continue;
+    const double* row = t1 + k * PS + I * N;
     double s = 0;
-    for (int J = 0; J < N; ++J) s += t1[(I * N + J) * kP + k] * H[1][J][j];
-    t2[(I * kP + j) * kP + k] = s;
+#pragma unroll 4
+    for (int J = 0; J < N; ++J) s += row[J] * H[1][J][j];
+    t2[t] = s;
   }
   __syncthreads();
-  // out[i][j][k] = cw sum_I t2[I][j][k] Hx[I][i]
-  for (int m = threadIdx.x; m < kModes; m += kThreads) {
+  // out[i][j][k] = cw sum_I t2[I][k][j] Hx[I][i]
+  for (int m = threadIdx.x; m < kModes; m += blockDim.x) {
     const int i = c_mi[m], j = c_mj[m], k = c_mk[m];
     double s = 0;
-    for (int I = 0; I < N; ++I) s += t2[(I * kP + j) * kP + k] * H[0][I][i];
+#pragma unroll 4
+    for (int I = 0; I < N; ++I) s += t2[(I * kP + k) * kP + j] * H[0][I][i];
     out[m] = s * a.cw;
   }
   __syncthreads();
@@ -208,34 +195,58 @@ __device__ void project_modes(const Field& g, int upt, int e, const FrameArgs& a
 // Features X[pt][256] (a_k of f - M, then sqrt(T)/L and u/L), frame
 // mom[pt][5], non-equilibrium measure eps[pt] = |a_k, degree >= 2|, and
 // optionally the targets B[pt][256] of a collision bank Q.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) embed_kernel(const T* __restrict__ f, const T* __restrict__ Q,
-                                                         const T* __restrict__ nu,
-                                                         FrameArgs a, float* __restrict__ X,
-                                                         float* __restrict__ B, double* __restrict__ mom_out,
-                                                         float* __restrict__ eps) {
+//
+// One CTA per point and one thread per row (I, J).  A point's values are 128
+// bytes apart in the bank, so a warp's load is 32 sectors whatever the order,
+// and what bounds the kernel is how many are in flight: each thread copies its
+// whole row to shared memory at once (cp.async) and takes both the moments and
+// the projection from there, and t1 then overlays the values.  576 points, N = 24,
+// FP32: 110 us (the L1's sectors 63 % busy) against 200 us with two passes over
+// the bank, a few loads in flight and 2.25 rows per thread.
+// STAGED = false (FP64 above N = 28, where the values do not fit): both read
+// the bank.
+template <typename T, bool STAGED, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) embed_kernel(const T* __restrict__ f, const T* __restrict__ Q,
+                                                              const T* __restrict__ nu,
+                                                              FrameArgs a, float* __restrict__ X,
+                                                              float* __restrict__ B, double* __restrict__ mom_out,
+                                                              float* __restrict__ eps) {
   extern __shared__ double sm[];
-  __shared__ double red[kThreads / 32];
+  __shared__ double red[kMaxN * kMaxN / 32];
   __shared__ double mom[5];
   __shared__ double H[3][kMaxN][kP];
   __shared__ double Ex[3][kMaxN];
   __shared__ double coef[kModes];
-  const int N = a.N;
-  double* t1 = sm;                    // [N*N][kP]
-  double* t2 = sm + N * N * kP;       // [N][kP][kP]
-  const int pt = blockIdx.x, upt = pt / a.neles, e = pt % a.neles;
+  const int N = a.N, NN = N * N;
+  double* const t2 = sm;                  // [N][kP][kP]
+  double* const t1 = sm + N * kP * kP;    // [kP][N*N + 1]
+  T* const sf = reinterpret_cast<T*>(t1); // [K][r] while it is read
+  const int pt = blockIdx.x, upt = pt / a.neles, e = pt % a.neles, r = threadIdx.x;
+  const long long b0 = dgfs::soa_ix(upt, a.ldim, e, (long long)r * N, (long long)NN * N, 32);
+  if (STAGED) {
+    if (r < NN) {
+      for (int K = 0; K < N; ++K)
+        __pipeline_memcpy_async(sf + K * NN + r, f + b0 + (long long)K * 32, sizeof(T));
+    }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);  // a thread reads its own row only
+  }
+  auto fval = [&](int K) -> double { return (double)(STAGED ? sf[K * NN + r] : f[b0 + (long long)K * 32]); };
 
   double m[5];
-  point_frame<T>(f, upt, e, a, red, m);
-  if (threadIdx.x < 5) mom[threadIdx.x] = m[threadIdx.x];
+  point_frame(fval, r, a, red, m);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) mom[k] = m[k];
+  }
   __syncthreads();
   basis_tables(a, mom, H, Ex);
   __syncthreads();
 
-  project_modes(DevField<T>{f}, upt, e, a, mom, H, Ex, t1, t2, coef);
+  project_modes([&](int K, double Mv) { return fval(K) - Mv; }, r, a, mom, H, Ex, t1, t2, coef);
   const double rho = mom[0];
   double ne = 0;
-  for (int k = threadIdx.x; k < kFeat; k += kThreads) {
+  for (int k = threadIdx.x; k < kFeat; k += blockDim.x) {
     float x = 0.f;
     if (k < kModes) {
       x = (float)(coef[k] / rho);
@@ -253,12 +264,19 @@ __global__ void __launch_bounds__(kThreads) embed_kernel(const T* __restrict__ f
     for (int k = 0; k < 5; ++k) mom_out[(long long)pt * 5 + k] = mom[k];
   }
   if (Q) {
+    // a bank value, or the gain deviation G - nu M = Q + nu (f - M)
+    const T* const q0 = Q + b0;
     if (nu)
-      project_modes(GainDevField<T>{Q, nu, f}, upt, e, a, mom, H, Ex, t1, t2, coef);
+      project_modes(
+          [&](int K, double Mv) {
+            const long long ix = (long long)K * 32;
+            return (double)q0[ix] + (double)nu[b0 + ix] * ((double)f[b0 + ix] - Mv);
+          },
+          r, a, mom, H, Ex, t1, t2, coef);
     else
-      project_modes(BankField<T>{Q}, upt, e, a, mom, H, Ex, t1, t2, coef);
+      project_modes([&](int K, double) { return (double)q0[(long long)K * 32]; }, r, a, mom, H, Ex, t1, t2, coef);
     const double s = 1.0 / (a.prefac * rho * rho * pow(mom[4], 0.5 * a.gamma));
-    for (int k = threadIdx.x; k < kFeat; k += kThreads)
+    for (int k = threadIdx.x; k < kFeat; k += blockDim.x)
       B[(long long)pt * kFeat + k] = k < kModes ? (float)(coef[k] * s) : 0.f;
   }
 }
@@ -449,6 +467,23 @@ __global__ void __launch_bounds__(kThreads) coef_kernel(const int* __restrict__ 
 // the projection and corrects its range.  The local Maxwellian comes from
 // per-point 1D Gaussian tables (the Gaussian factorises over the axes).
 
+// A thread's loads of kRelaxBatch nodes are issued together (one node at a time
+// left each warp with an L2 round trip per node; 576 points, N = 24, FP32:
+// pass 1 66 -> 50 us, pass 2 44 -> 33 us).
+constexpr int kRelaxBatch = 9;
+
+// the velocity kRelaxWarps nodes on: carry K into J into I
+__device__ __forceinline__ void advance(int N, int& I, int& J, int& K) {
+  K += kRelaxWarps;
+  while (K >= N) {
+    K -= N;
+    if (++J == N) {
+      J = 0;
+      ++I;
+    }
+  }
+}
+
 struct RelaxPoint {
   int upt, eb, lane, e;
 };
@@ -501,26 +536,29 @@ __global__ void __launch_bounds__(kRelaxWarps * 32) relax_pass1_kernel(const dou
     const double msc = ms[P.lane];
     const long long base = (long long)P.upt * a.ldim + (long long)P.eb * V * 32 + P.lane;
     int I = (v0 + w) / (N * N), J = ((v0 + w) / N) % N, K = (v0 + w) % N;
-#pragma unroll 4
-    for (int v = v0 + w; v < v1; v += kRelaxWarps) {
-      const long long ix = base + (long long)v * 32;
-      const double M = msc * Ex[P.lane][I] * Ex[P.lane][N + J] * Ex[P.lane][2 * N + K];
-      const double q = -(double)nu[ix] * ((double)f[ix] - M);
-      Q[ix] = (T)q;
-      const double cx = c00 + I * h, cy = c00 + J * h, cz = c00 + K * h;
-      m[0] += q;
-      m[1] += q * cx;
-      m[2] += q * cy;
-      m[3] += q * cz;
-      m[4] += q * (cx * cx + cy * cy + cz * cz);
-      // next v: carry K into J into I
-      K += kRelaxWarps;
-      while (K >= N) {
-        K -= N;
-        if (++J == N) {
-          J = 0;
-          ++I;
-        }
+    for (int vb = v0 + w; vb < v1; vb += kRelaxBatch * kRelaxWarps) {
+      T fb[kRelaxBatch], nb[kRelaxBatch];
+#pragma unroll
+      for (int p = 0; p < kRelaxBatch; ++p) {
+        const int v = vb + p * kRelaxWarps;
+        const long long ix = base + (long long)v * 32;
+        fb[p] = v < v1 ? f[ix] : T(0);
+        nb[p] = v < v1 ? nu[ix] : T(0);
+      }
+#pragma unroll
+      for (int p = 0; p < kRelaxBatch; ++p) {
+        const int v = vb + p * kRelaxWarps;
+        if (v >= v1) break;
+        const double M = msc * Ex[P.lane][I] * Ex[P.lane][N + J] * Ex[P.lane][2 * N + K];
+        const double q = -(double)nb[p] * ((double)fb[p] - M);
+        Q[base + (long long)v * 32] = (T)q;
+        const double cx = c00 + I * h, cy = c00 + J * h, cz = c00 + K * h;
+        m[0] += q;
+        m[1] += q * cx;
+        m[2] += q * cy;
+        m[3] += q * cz;
+        m[4] += q * (cx * cx + cy * cy + cz * cz);
+        advance(N, I, J, K);
       }
     }
   }
@@ -571,18 +609,21 @@ __global__ void __launch_bounds__(kRelaxWarps * 32) relax_pass2_kernel(const int
                l4 = lam[P.lane][4];
   const long long base = (long long)P.upt * a.ldim + (long long)P.eb * V * 32 + P.lane;
   int I = (v0 + w) / (N * N), J = ((v0 + w) / N) % N, K = (v0 + w) % N;
-#pragma unroll 4
-  for (int v = v0 + w; v < v1; v += kRelaxWarps) {
-    const long long ix = base + (long long)v * 32;
-    const double cx = c00 + I * h, cy = c00 + J * h, cz = c00 + K * h;
-    Q[ix] = (T)((double)Q[ix] - (l0 + l1 * cx + l2 * cy + l3 * cz + l4 * (cx * cx + cy * cy + cz * cz)));
-    K += kRelaxWarps;
-    while (K >= N) {
-      K -= N;
-      if (++J == N) {
-        J = 0;
-        ++I;
-      }
+  for (int vb = v0 + w; vb < v1; vb += kRelaxBatch * kRelaxWarps) {
+    T qb[kRelaxBatch];
+#pragma unroll
+    for (int p = 0; p < kRelaxBatch; ++p) {
+      const int v = vb + p * kRelaxWarps;
+      qb[p] = v < v1 ? Q[base + (long long)v * 32] : T(0);
+    }
+#pragma unroll
+    for (int p = 0; p < kRelaxBatch; ++p) {
+      const int v = vb + p * kRelaxWarps;
+      if (v >= v1) break;
+      const double cx = c00 + I * h, cy = c00 + J * h, cz = c00 + K * h;
+      Q[base + (long long)v * 32] =
+          (T)((double)qb[p] - (l0 + l1 * cx + l2 * cy + l3 * cz + l4 * (cx * cx + cy * cy + cz * cz)));
+      advance(N, I, J, K);
     }
   }
 }
@@ -662,17 +703,28 @@ extern "C" int dgfs_hermite_embed(int precision, const void* f, const void* Q, c
   if (!rc) rc = init_modes();
   if (rc) return rc;
   FrameArgs a{Nv, nupts, neles, ldim, L, cw, prefactor, gamma};
-  const size_t smem = ((size_t)Nv * Nv * kP + (size_t)Nv * kP * kP) * sizeof(double);
-  const void* fn = precision == 64 ? (const void*)embed_kernel<double> : (const void*)embed_kernel<float>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return dgfs::set_error(DGFS_ERR_CUDA, "smem attribute");
-  const unsigned grid = (unsigned)(nupts * neles);
-  if (precision == 64)
-    embed_kernel<double><<<grid, kThreads, smem, (cudaStream_t)stream>>>((const double*)f, (const double*)Q,
-                                                                          (const double*)nu, a, X, B, mom, eps);
-  else
-    embed_kernel<float><<<grid, kThreads, smem, (cudaStream_t)stream>>>((const float*)f, (const float*)Q,
-                                                                         (const float*)nu, a, X, B, mom, eps);
+  const size_t vals = (size_t)Nv * Nv * Nv * (precision / 8), t1 = (size_t)(Nv * Nv + 1) * kP * sizeof(double),
+               t2 = (size_t)Nv * kP * kP * sizeof(double);
+  // staged where the values fit beside 12 KB of tables (all of FP32, FP64 to N = 28)
+  const bool staged = std::max(vals, t1) + t2 <= (227 - 12) * 1024;
+  const size_t smem = (staged ? std::max(vals, t1) : t1) + t2;
+  const unsigned grid = (unsigned)(nupts * neles), nt = (unsigned)((Nv * Nv + 31) / 32 * 32);
+  auto launch = [&](auto* kernel, auto* fb) {
+    using T = std::remove_pointer_t<decltype(fb)>;
+    if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return false;
+    kernel<<<grid, nt, smem, (cudaStream_t)stream>>>(fb, (T*)Q, (T*)nu, a, X, B, mom, eps);
+    return true;
+  };
+  // up to N = 24 in FP32 two CTAs share an SM (56 registers a thread)
+  constexpr int kMid = 24 * 24, kMax = kMaxN * kMaxN;
+  const bool ok = precision == 32
+                      ? (nt <= kMid ? launch(embed_kernel<float, true, kMid, 2>, (const float*)f)
+                                    : launch(embed_kernel<float, true, kMax, 1>, (const float*)f))
+                  : staged ? launch(embed_kernel<double, true, kMax, 1>, (const double*)f)
+                           : launch(embed_kernel<double, false, kMax, 1>, (const double*)f);
+  if (!ok) return dgfs::set_error(DGFS_ERR_CUDA, "smem attribute");
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return dgfs::set_error(DGFS_ERR_CUDA, "embed launch: %s", cudaGetErrorString(e));
   return DGFS_OK;

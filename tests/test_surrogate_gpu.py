@@ -530,3 +530,38 @@ def test_scale_rows_matches_numpy():
         _lib.check(lib.dgfs_surrogate_scale(M, NFEAT, d_e.data_ptr(), 1e-3,
                                             0, NMODES, 10, 0, d_x.data_ptr(),
                                             s), 'dgfs_surrogate_scale')
+
+
+@pytest.mark.parametrize('precision,Nv', [
+    ('single', 8), ('single', 16), ('single', 24), ('single', 32),
+    ('double', 8), ('double', 16), ('double', 24), ('double', 32)])
+def test_embed_at_every_staging_size(precision, Nv):
+    """Values smaller and larger than the table that overlays them, both
+    register budgets, and FP64 values that do not fit and are read from the
+    bank; the second call finds the same results.  Tolerances as above: FP64
+    sums, coefficients stored in FP32."""
+    cfg = config('channel-n32', precision, Nv=Nv, Nrho=2, M=6)
+    be = B200Backend(cfg, device='cuda:0')
+    vm = DGFSVelocityMesh(be, cfg)
+    sm = DGFSVHSGLLScatteringModel(be, cfg, vm)
+    cv, cw = vm.cv(), vm.cw()
+    nupts, neles = 1, 3
+    f = random_states(cv, neles, seed=Nv).reshape(nupts, neles, -1)
+    q = random_states(cv, neles, seed=Nv + 1).reshape(nupts, neles, -1)
+    fb, qb = _bank(be, f), _bank(be, q)
+    sur = VHSSurrogate(sm)
+    first = sur.embed(fb, qb)
+    again = sur.embed(fb, qb)
+    torch.cuda.synchronize()
+    for a, b in zip(first, again):
+        assert torch.equal(a, b)
+    X, B, mom, eps = (t.cpu().numpy() for t in first)
+    fu, qu = fb.get().astype(np.float64), qb.get().astype(np.float64)
+    for e in range(neles):
+        x, (rho, uu, T), ep, b = osur.embed(
+            fu[0, :, e], cv, cw, vm.L(), Q=qu[0, :, e], prefac=sm.prefactor,
+            gamma=sm._gamma)
+        assert rel_err(mom[e], np.r_[rho, uu, T]) < 1e-12
+        assert rel_err(X[e], x) < 1e-5
+        assert rel_err(B[e], b) < 1e-5
+        assert abs(eps[e] - ep) < 1e-5*ep
