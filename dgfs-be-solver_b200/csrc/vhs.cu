@@ -2,6 +2,7 @@
 // precomputed tables of frfs's perform_precomputation
 // (frfs/solvers/dgfs/scattering.py:67-224, vhs-gll.mako:45-101) and the
 // cluster-kernel dispatch behind the C ABI in include/dgfs_b200.h.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -181,9 +182,9 @@ struct dgfs_vhs {
   double* cvec;  // [3][V]
   void* fc;      // scratch: gain spectrum, one N^3 complex slice per cluster
   size_t fc_bytes;
-  void* fcp;     // single-CTA kernel: partial gain spectra of split points (kCubeSlices per CTA)
+  void* fcp;     // single-CTA kernel: partial gain spectra of split points (kCubeSlices or P per CTA)
   size_t fcp_bytes;
-  int* pdone;    // ... and the chunk counters (kCubeSlices / 2 per CTA, zero between launches)
+  int* pdone;    // ... and the chunk counters (one per CTA, zero between launches)
   int pdone_n;
   int* err;      // device flag: a bounded wait in the kernel gave up
 };
@@ -240,11 +241,10 @@ static int select_index(dgfs_vhs* h, int idx) {
     h->fc_bytes = need;
   }
   if (v->push == 2) {
-    // a launch on few points splits them into radial-node chunks: up to
-    // kCubeSlices items per CTA, each with its own partial-spectrum slice,
-    // and (at least 2 chunks per point) up to kCubeSlices / 2 points per CTA
-    // with a chunk counter
-    const size_t needp = (size_t)kCubeSlices * ncl * v->slice_cx * esz;
+    // a launch on few points (no more than CTAs) splits them into P
+    // radial-node chunks: up to kCubeSlices items per CTA, each with its own
+    // partial-spectrum slice, and a chunk counter per point
+    const size_t needp = (size_t)std::min(kCubeSlices, h->P) * ncl * v->slice_cx * esz;
     if (needp > h->fcp_bytes) {
       cudaFree(h->fcp);
       h->fcp = nullptr;
@@ -253,7 +253,7 @@ static int select_index(dgfs_vhs* h, int idx) {
         return set_error(DGFS_ERR_NOMEM, "cudaMalloc(%zu) for the partial-spectrum scratch failed", needp);
       h->fcp_bytes = needp;
     }
-    const int npd = kCubeSlices / 2 * ncl;
+    const int npd = ncl;
     if (npd > h->pdone_n) {
       cudaFree(h->pdone);
       h->pdone = nullptr;

@@ -114,10 +114,12 @@ template <typename T, int N> struct CubeGeom {
 // P chunks: with one node per chunk the final sum over the chunks' slices
 // adds the nodes in the same order as the unsplit accumulation, so a point's
 // Q does not depend on the launch it is part of (bit for bit).  Items are
-// capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch).
+// capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch), and
+// more points than CTAs are not split (N = 24: 160 points 2,240 us split, 2,103
+// us whole).
 // Every CTA computes the same value.
 __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
-  if (P < 2 || (long long)npts * P > (long long)kCubeSlices * G) return 1;
+  if (P < 2 || npts > G || (long long)npts * P > (long long)kCubeSlices * G) return 1;
   constexpr double kFixed = 48.0;
   const double per_node = 3.0 * M + 3.0;
   const double whole = (double)((npts + G - 1) / G) * (P * per_node + kFixed);

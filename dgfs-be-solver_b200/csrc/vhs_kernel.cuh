@@ -61,7 +61,7 @@ template <typename T> struct VhsArgs {
   cx<T>* fcp;           // single-CTA kernel, points split over CTAs: partial gain
                         // spectra, one [V] slice per (point, radial chunk) item
                         // (<= kCubeSlices gridDim.x)
-  int* pdone;           // ... and per point the chunks finished (<= kCubeSlices / 2 gridDim.x points;
+  int* pdone;           // ... and per point the chunks finished (<= gridDim.x points;
                         // zero between launches).  NULL: never split.
   int* err;             // set to 1 when a bounded wait gives up
   const int* plist;     // optional device list of linear points (NULL: pt0 + i)

@@ -22,7 +22,7 @@ struct VhsVariant {
 
 // partial-spectrum slices per CTA of the single-CTA kernel: a launch on few
 // points splits them into one work item per radial node, at most so many per
-// CTA of the grid (with P = 12 up to two waves of whole points)
+// CTA of the grid
 constexpr int kCubeSlices = 24;
 
 // single-CTA kernel (kind 2 in dgfs_vhs_variant_kind): FP32 N = 8, 16, 24 and
