@@ -759,6 +759,8 @@ class VHSSurrogate:
             self._side_nu = torch.cuda.Stream(device=self.device)
             self._fork = torch.cuda.Event()
             self._join = torch.cuda.Event()
+        # made before the fork, on the stream whose memory pool it lives in
+        nubank = self.nu_bank(fbank)
         self._fork.record(main)
         self._side.wait_event(self._fork)
         _lib.check(lib.dgfs_vhs_apply_list(
@@ -770,7 +772,7 @@ class VHSSurrogate:
         # both need nothing but the gate: side by side
         self._side_nu.wait_event(self._fork)
         with torch.cuda.stream(self._side_nu):
-            nu = self.loss_rate(fbank, self.nu_bank(fbank), gate)
+            nu = self.loss_rate(fbank, nubank, gate)
         Bp = self.scale_targets(self.predict(X, net, nnet), eps,
                                 inverse=True)
         main.wait_stream(self._side_nu)
