@@ -565,3 +565,32 @@ def test_embed_at_every_staging_size(precision, Nv):
         assert rel_err(X[e], x) < 1e-5
         assert rel_err(B[e], b) < 1e-5
         assert abs(eps[e] - ep) < 1e-5*ep
+
+
+@pytest.mark.parametrize('precision,Nv', [
+    ('single', 8), ('single', 16), ('single', 24), ('single', 32),
+    ('double', 16), ('double', 24)])
+def test_loss_rate_of_neighbouring_elements(precision, Nv):
+    """An element's collision frequency does not depend on the neighbour it
+    shares a CTA with, on a neighbour that is gated off, or on being the last
+    of an odd number; gated-off points keep what they hold (bit for bit: the
+    values themselves are compared with the oracle above)."""
+    cfg = config('channel-n32', precision, Nv=Nv, Nrho=2, M=6)
+    be = B200Backend(cfg, device='cuda:0')
+    vm = DGFSVelocityMesh(be, cfg)
+    sm = DGFSVHSGLLScatteringModel(be, cfg, vm)
+    sur = VHSSurrogate(sm)
+    neles = 35
+    f = random_states(vm.cv(), neles + 1, seed=Nv)
+    whole = _bank(be, f[None, :neles])
+    shifted = _bank(be, f[None, 1:])
+    a = sur.loss_rate(whole, be.matrix(whole.ioshape)).get()[0]
+    b = sur.loss_rate(shifted, be.matrix(shifted.ioshape)).get()[0]
+    assert np.array_equal(a[:, 1:], b[:, :-1])
+    gate = torch.zeros(neles, dtype=torch.int32, device=be.device)
+    on = [0, 3, 6, 7, 34]
+    gate[on] = 1
+    out = be.matrix(whole.ioshape, np.full(whole.ioshape, 7.0))
+    c = sur.loss_rate(whole, out, gate).get()[0]
+    off = [e for e in range(neles) if e not in on]
+    assert np.array_equal(c[:, on], a[:, on]) and np.all(c[:, off] == 7.0)
