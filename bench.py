@@ -53,17 +53,17 @@ METRIC = 'Q(f) evals/s'
 # (kernel, workload, points, precision bits) -> (bytes, how it was taken)
 TRAFFIC = {
     ('vhs_cube_kernel', 'couette-n24', 576, 32):
-        (36.7e6, 'captured at this size'),
+        (35.4e6, 'captured at this size'),
     ('vhs_pair_kernel', 'channel-n32', 10368, 32):
-        (208.3e6*72, 'captured on the 4 x 4-element channel (144 points, '
-                     '208.3 MB, 512-thread layout) and scaled by the point '
+        (192.9e6*72, 'captured on the 4 x 4-element channel (144 points, '
+                     '192.9 MB, 608-thread layout) and scaled by the point '
                      'count (x72)'),
 }
 # the same for one DG stage (interp + residual): (workload, points, bits)
 DG_TRAFFIC = {
     ('couette-n24', 576, 32):
-        (148.9e6, 'captured at this size (interp 33.5 MB + residual '
-                  '115.4 MB, residual shape of 8 velocities per warp)'),
+        (190.1e6, 'captured at this size (interp 32.7 MB + residual '
+                  '157.4 MB, residual shape of 4 velocities per warp)'),
 }
 
 
@@ -724,7 +724,7 @@ def run_b200(args):
                                'dram__bytes_write.sum: ' + dg_tsrc)
             if dg_traffic else 'not captured for this workload/size/'
                                'precision',
-            'kernels': 'dg_interp_kernel + dg_residual_kernel',
+            'kernels': 'dg_interp_fac_kernel + dg_residual_fac_kernel',
             'residual_shape': system.dg_variants()[system._dg_shape],
             'ms_by_shape': dg_tune}
     launch = sm.launch_info()

@@ -242,7 +242,9 @@ DGFS_API int dgfs_vss_status(dgfs_vss* h, void* stream, int* flag);
 /* No counterpart in the reference: the launch shape of a handle.  pair = 1
  * selects the two-CTA kernel (FP32, Nv = 24; the default there), pair = 0
  * the cluster exchange kernel.  DGFS_ERR_UNSUPPORTED when the shape does
- * not exist for the handle's precision and Nv. */
+ * not exist for the handle's precision and Nv.  The first pair = 0 on a
+ * handle with the two-CTA kernel allocates that kernel's order of the gain
+ * tables (DGFS_ERR_NOMEM): not under capture. */
 DGFS_API int dgfs_vss_select(dgfs_vss* h, int pair);
 
 /* ------------------------------------------------------------------------
