@@ -229,4 +229,188 @@ template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[
   }
 }
 
+// ---- FP32 transforms of the VHS collision kernels ------------------------------
+//
+//   mfft<N, S>(x), N = 8 Q, Q = 1 .. 4: 8 points (4 x 2), one layer of
+//   twiddles, Q points
+//
+// the mixed-radix transform of fft_reg.cuh operation by operation, on packed
+// values: every sum, product and fused product is rounded where that
+// transform rounds it, so the results are its results bit for bit.  The
+// collision kernels take it in FP32 because Q near equilibrium is the small
+// difference of gain and loss (1e-4 of either at a distance of 1e-2) and shows
+// the transforms' round-off: with cfft above, whose N = 32 has two layers of
+// rounded twiddles, the error of Q rose by a factor 1.26 at N = 32; with cfft<24>
+// it fell by 0.78 at N = 24, but at a distance of 1e-2 either change is percents
+// of Q.
+//
+//   mfft_scaled<N, S>(x, m): the same of x[k] m(k), real factors: the products
+//   of the first butterflies' leading terms are fused into their sums.
+
+// cos(2 pi j / 96), j <= 24
+__host__ __device__ constexpr double cos96(int j) {
+  constexpr double c[25] = {
+      1.0, 0.99785892323860350673, 0.99144486137381041114, 0.98078528040323044912, 0.96592582628906828674,
+      0.94693012949510566425, 0.92387953251128675612, 0.89687274153268830389, 0.86602540378443864676,
+      0.83146961230254523707, 0.79335334029123516457, 0.75183980747897739640, 0.70710678118654752440,
+      0.65934581510006886842, 0.60876142900872063941, 0.55557023301960222474, 0.5, 0.44228869021900128199,
+      0.38268343236508977172, 0.32143946530316158070, 0.25881904510252076234, 0.19509032201612826784,
+      0.13052619222005159154, 0.06540312923014306681, 0.0};
+  j = j < 0 ? -j : j;
+  j %= 96;
+  j = j > 48 ? 96 - j : j;
+  return j > 24 ? -c[48 - j] : c[j];
+}
+// i S a
+template <int S> __device__ __forceinline__ cpx rot_i(cpx a) {
+  return S > 0 ? cpk(-cim(a), cre(a)) : cpk(cim(a), -cre(a));
+}
+// a exp(S 2 pi i m / N)
+template <int N, int S, int m> __device__ __forceinline__ cpx mtwiddle(cpx a) {
+  constexpr int mm = m % N;
+  if constexpr (mm == 0) {
+    return a;
+  } else if constexpr (2 * mm == N) {
+    return cpk(-cre(a), -cim(a));
+  } else if constexpr (4 * mm == N) {
+    return rot_i<S>(a);
+  } else if constexpr (4 * mm == 3 * N) {
+    return rot_i<-S>(a);
+  } else {
+    constexpr float c = (float)cos96(mm * (96 / N)), s = S * (float)cos96(mm * (96 / N) - 24);
+    return cpk(fmaf(cre(a), c, -__fmul_rn(cim(a), s)), fmaf(cim(a), c, __fmul_rn(cre(a), s)));
+  }
+}
+
+// the rest of an 8-point transform whose two 4-point ones are done:
+// e = transform of the even, o of the odd inputs (o[2] with its parts swapped)
+template <int S> __device__ __forceinline__ void mfft8_join(const cpx (&e)[4], const cpx (&o)[4], cpx (&t)[8]) {
+  t[0] = vadd(e[0], o[0]);
+  t[4] = vsub(e[0], o[0]);
+  const cpx w1 = mtwiddle<8, S, 1>(o[1]), w3 = mtwiddle<8, S, 3>(o[3]);
+  t[1] = vadd(e[1], w1);
+  t[5] = vsub(e[1], w1);
+  t[2] = add_rot<S, 0>(e[2], o[2]);
+  t[6] = add_rot<-S, 0>(e[2], o[2]);
+  t[3] = vadd(e[3], w3);
+  t[7] = vsub(e[3], w3);
+}
+
+// outputs of the 8-point transforms t[q] of x[Q r + q], through the twiddles
+// and the Q-point transforms
+template <int N, int S> __device__ __forceinline__ void mfft_join(cpx (&t)[N / 8][8], cpx (&x)[N]) {
+  constexpr int Q = N / 8;
+  sfor<0, 8>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    if constexpr (Q == 1) {
+      x[k] = t[0][k];
+    } else if constexpr (Q == 2) {
+      const cpx b = mtwiddle<N, S, k>(t[1][k]);
+      x[k] = vadd(t[0][k], b);
+      x[k + 8] = vsub(t[0][k], b);
+    } else if constexpr (Q == 3) {
+      const cpx a = t[0][k], b = mtwiddle<N, S, k>(t[1][k]), c = mtwiddle<N, S, 2 * k>(t[2][k]);
+      const cpx s = vadd(b, c), ds = sub_swap(b, c), e = sub_half(a, s);
+      x[k] = vadd(a, s);
+      x[k + 8] = add_rot<S, 1>(e, ds);
+      x[k + 16] = add_rot<-S, 1>(e, ds);
+    } else {
+      cpx a = t[0][k], b = mtwiddle<N, S, k>(t[1][k]), c = mtwiddle<N, S, 2 * k>(t[2][k]),
+          d = mtwiddle<N, S, 3 * k>(t[3][k]);
+      cfft4<S, false>(a, b, c, d);
+      x[k] = a;
+      x[k + 8] = b;
+      x[k + 16] = c;
+      x[k + 24] = d;
+    }
+  });
+}
+
+template <int N, int S> __device__ __forceinline__ void mfft(cpx (&x)[N]) {
+  constexpr int Q = N / 8;
+  static_assert(N % 8 == 0 && Q >= 1 && Q <= 4, "8 Q points");
+  cpx t[Q][8];
+  sfor<0, Q>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    cpx e[4] = {x[q], x[q + 2 * Q], x[q + 4 * Q], x[q + 6 * Q]};
+    cpx o[4] = {x[q + Q], x[q + 3 * Q], x[q + 5 * Q], x[q + 7 * Q]};
+    cfft4<S, false>(e[0], e[1], e[2], e[3]);
+    cfft4<S, true>(o[0], o[1], o[2], o[3]);
+    mfft8_join<S>(e, o, t[q]);
+  });
+  mfft_join<N, S>(t, x);
+}
+
+// cfft4 of a m0, b m1, c m2, d m3.  Scalar: a packed factor (m, m) costs a move
+template <int S, bool SW>
+__device__ __forceinline__ void mfft4_scaled(cpx& a, cpx& b, cpx& c, cpx& d, float m0, float m1, float m2, float m3) {
+  const float p2x = __fmul_rn(cre(c), m2), p2y = __fmul_rn(cim(c), m2);
+  const float p3x = __fmul_rn(cre(d), m3), p3y = __fmul_rn(cim(d), m3);
+  const cpx s0 = cpk(fmaf(cre(a), m0, p2x), fmaf(cim(a), m0, p2y));
+  const cpx d0 = cpk(fmaf(cre(a), m0, -p2x), fmaf(cim(a), m0, -p2y));
+  const cpx s1 = cpk(fmaf(cre(b), m1, p3x), fmaf(cim(b), m1, p3y));
+  const cpx d1 = cpk(fmaf(cim(b), m1, -p3y), fmaf(cre(b), m1, -p3x));  // parts swapped
+  a = vadd(s0, s1);
+  if constexpr (SW) c = sub_swap(s0, s1);
+  else c = vsub(s0, s1);
+  b = add_rot<S, 0>(d0, d1);
+  d = add_rot<-S, 0>(d0, d1);
+}
+
+template <int N, int S, typename M> __device__ __forceinline__ void mfft_scaled(cpx (&x)[N], const M& m) {
+  constexpr int Q = N / 8;
+  static_assert(N % 8 == 0 && Q >= 1 && Q <= 4, "8 Q points");
+  cpx t[Q][8];
+  sfor<0, Q>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    cpx e[4] = {x[q], x[q + 2 * Q], x[q + 4 * Q], x[q + 6 * Q]};
+    cpx o[4] = {x[q + Q], x[q + 3 * Q], x[q + 5 * Q], x[q + 7 * Q]};
+    mfft4_scaled<S, false>(e[0], e[1], e[2], e[3], m(q), m(q + 2 * Q), m(q + 4 * Q), m(q + 6 * Q));
+    mfft4_scaled<S, true>(o[0], o[1], o[2], o[3], m(q + Q), m(q + 3 * Q), m(q + 5 * Q), m(q + 7 * Q));
+    mfft8_join<S>(e, o, t[q]);
+  });
+  mfft_join<N, S>(t, x);
+}
+
+// ---- the collision kernels' lines in either precision ---------------------------
+template <int N, int S> __device__ __forceinline__ void vfft(cpx (&x)[N]) { mfft<N, S>(x); }
+template <int N, int S> __device__ __forceinline__ void vfft(double2 (&x)[N]) { cfft<N, S>(x); }
+template <int N, int S, typename M> __device__ __forceinline__ void vfft_scaled(cpx (&x)[N], const M& m) {
+  mfft_scaled<N, S>(x, m);
+}
+template <int N, int S, typename M> __device__ __forceinline__ void vfft_scaled(double2 (&x)[N], const M& m) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double f = m(k);
+    x[k] = make_double2(x[k].x * f, x[k].y * f);
+  }
+  cfft<N, S>(x);
+}
+// a b, and a (1 - b), with the roundings of FP32 stated (which of the two
+// products is rounded by itself is the compiler's choice otherwise)
+__device__ __forceinline__ float2 mul_r(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ float2 mul_1m(float2 a, float2 b) {
+  const float c = 1.f - b.x;
+  return make_float2(fmaf(a.y, b.y, __fmul_rn(a.x, c)), fmaf(a.y, c, -__fmul_rn(a.x, b.y)));
+}
+// a + a b, from ab: its imaginary part's other product is the rounded one
+__device__ __forceinline__ float2 mul_s(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ double2 mul_r(double2 a, double2 b) { return cmul(a, b); }
+__device__ __forceinline__ double2 mul_s(double2 a, double2 b) { return cmul(a, b); }
+__device__ __forceinline__ double2 mul_1m(double2 a, double2 b) { return cmul(a, make_double2(1.0 - b.x, -b.y)); }
+// Re(a b)
+__device__ __forceinline__ float re_mul(float2 a, float2 b) { return fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ double re_mul(double2 a, double2 b) { return a.x * b.x - a.y * b.y; }
+// s + Re r^2 + Re n^2 (FP32), or s + Re r Im r + Re n Im n: the same of r and n
+// made from (1 + i) F (FP64)
+__device__ __forceinline__ float add_squares(cpx r, cpx n, float s) {
+  const float v = fmaf(cre(r), cre(r), -__fmul_rn(cim(r), cim(r)));
+  return __fadd_rn(s, fmaf(-cim(n), cim(n), fmaf(cre(n), cre(n), v)));
+}
+__device__ __forceinline__ double add_squares(double2 r, double2 n, double s) { return fma(r.x, r.y, fma(n.x, n.y, s)); }
+
 }  // namespace dgfs

@@ -26,21 +26,23 @@
 // instead of two.  Per point: 1 + Nrho M + Nrho + 2 full transforms plus
 // the 2D ones (reference: 3 Nrho M + 3).
 //
-// One more restatement, also exact: with P = (1 + i) R, Re R^2 = Re P Im P
-// (and Re Nq^2 likewise), so the kernel transforms F^ = (1 + i) F and
-// accumulates one product per field.
+// FP64 restates it once more, also exactly: with P = (1 + i) R, Re R^2 =
+// Re P Im P (and Re Nq^2 likewise), so it transforms F^ = (1 + i) F and
+// accumulates one product per field.  FP32 keeps F^ = F and the squares, and
+// the mixed-radix transforms, in a fixed order of roundings (fft_vec.cuh): near
+// equilibrium Q is 1e-6 to 1e-2 of the gain, and what is left of it depends on
+// that order.
 //
-// What bounds it: shared memory and the FP32 pipe, each about half busy, and
-// the passes' latencies.  Per (p, q) the work cube crosses shared memory four
-// times (two exchanges) and every complex value takes about 13 operations a
-// pass.  So: a thread owns one line (N = 24: 18 warps and 2 for the Nyquist
-// planes, five per scheduler; nine warps with two lines per thread left one
-// scheduler with half as many again as the others), in packed FP32 registers
-// (fft_vec.cuh: half the issue slots); everything that only its own thread
-// touches -- the spectrum line F^ and the sums S_p -- lives in tensor memory,
-// which costs neither registers nor shared-memory bandwidth (two lines per
-// thread with S_p in registers spilled: 5.7 ms a sweep, 4.7 ms with S_p in
-// tensor memory); and no shared access of the main threads conflicts.
+// What bounds it: shared memory, the FP32 pipe and the passes' latencies.  Per
+// (p, q) the work cube crosses shared memory four times (two exchanges) and
+// every complex value takes 13 to 16 operations a pass.  So: a thread owns one
+// line (N = 24: 18 warps and 2 for the Nyquist planes, five per scheduler; nine
+// warps with two lines per thread left one scheduler with half as many again as
+// the others), in FP32 as packed registers (fft_vec.cuh: sums and differences
+// in half the issue slots); everything that only its own thread
+// touches -- the spectrum line and the sums S_p -- lives in tensor memory,
+// which costs neither registers nor shared-memory bandwidth; and no shared
+// access of the main threads conflicts.
 //
 // Layout in shared memory (complex float):
 //   sW   work cube: line (k1, k2) at k1 PS + off(k2), off(k) = N k + (k >= N/2).
@@ -48,21 +50,21 @@
 //        second 8 planes x {x3, x3 + 1}, of the third 8 x3 x {x2, x2 + N/2}:
 //        16 distinct 8-byte banks each (FP64: 8 lanes, 8 16-byte banks)
 //   sT1 [x2][x3], sT2 [x1][x3], sT3 [x2][x1]: the transformed Nyquist planes
-//   sN   [k][line] F^ on the Nyquist planes; sX their first axis
+//   sN   [k][line] the spectrum on the Nyquist planes; sX their first axis
 //   phases of (p, q) and of the next, in two slots
 // The main threads are N/8 groups, each owning 8 planes k1: the second pass of
 // a group needs only that group's first pass, so groups synchronise among
 // themselves.  The third pass releases the cube as soon as its values are in
 // registers, so its arithmetic runs beside the next first pass.  NQ more
-// threads transform the Nyquist planes and fetch the next phases.  S_p is real, so the gain spectrum is kept for k1 <= N/2, in a global
-// (L2-resident) slice per CTA, [k3][line].
+// threads transform the Nyquist planes and fetch the next phases.  The gain
+// spectrum is kept in a global (L2-resident) slice per CTA, [k3][line].
 //
-// Measured on one B200 (FP32, N = 24, 12 x 16 (p, q), 576 points): 4.16 ms a
-// sweep against 5.16 ms for the two-lines-per-thread kernel with scalar
-// transforms that this one replaces; FP32 pipe 48 % busy, shared memory 6.0K of
-// 9.9K cycles per (p, q).  N = 16 (8 x 6): 592 points 0.485 ms against 1.16 ms
-// for the two-CTA push kernel; FP64 N = 16, one point 71 us against 204 us
-// (its radial nodes spread over the SMs).
+// Measured on one B200 (FP32, N = 24, 12 x 16 (p, q), 576 points): 4.76 ms a
+// sweep against 5.17 ms for two lines per thread with scalar transforms, with
+// the same roundings.  N = 16 (8 x 6): FP64, one point 59 us against 191 us for
+// the two-CTA push kernel (its radial nodes spread over the SMs); FP32, 592
+// points 0.53 ms against 1.16 ms, but its error is 1.2 times that of the push
+// kernel's two transforms per (p, q), so there it is not the default.
 #pragma once
 
 #include "fft_vec.cuh"
@@ -80,7 +82,9 @@ template <typename T, int N> struct CubeGeom {
   static constexpr int NT = NM + NQ;
   static constexpr int PS = NN + (sizeof(T) == 4 ? 2 : 1);  // plane stride of the work cube
   static constexpr int PHS = 3 * N + 4;              // one phase slot
-  static constexpr int NL = H * N;                   // lines of the gain spectrum (k1 <= N/2)
+  // FP64 keeps the gain spectrum for k1 <= N/2 (the transform of a real S_p),
+  // FP32 all of it: mirrored values differ from transformed ones by round-off
+  static constexpr int GK = sizeof(T) == 4 ? N : H, NL = GK * N;  // lines of the gain spectrum
   static constexpr int SL = NL * N;                  // gain spectrum slice (complex)
   // tensor memory columns: per main warp 2 N values of F^, then N of S
   static constexpr int WD = sizeof(T) / 4;           // columns per value
@@ -105,18 +109,16 @@ template <typename T, int N> struct CubeGeom {
 // (3 M + 3) + kFixed) passes.  kFixed is what an item costs before its first
 // node and after its last (its own transform of f, the tables, the slice and
 // the point's last pass), fitted from the time per wave of split and of whole
-// items: 59 passes at N = 24 (P = 12, M = 16: 172 against 1,048 us a wave),
-// 48 at N = 16 FP32 (P = 8, M = 6: 38 against 117 us) and 43 in FP64 (56
-// against 185 us).  So a split pays up to 6, 3 and 3 waves: 74 points at
-// N = 24 take 1,048 us split and 1,062 us whole, 98 points 1,390 against 1,062 us;
-// 49 at N = 16 take 125 against 131 us (FP64 182 against 201 us), 61 points
-// 163 against 131 us (239 against 201 us).  Only 1 or
-// P chunks: with one node per chunk the final sum over the chunks' slices
-// adds the nodes in the same order as the unsplit accumulation, so a point's
-// Q does not depend on the launch it is part of (bit for bit).  Items are
-// capped at kCubeSlices per CTA of the grid (the partial-spectrum scratch), and
-// more points than CTAs are not split (N = 24: 160 points 2,240 us split, 2,103
-// us whole).
+// items: 62 passes at N = 24 (P = 12, M = 16: 200 against 1,194 us a wave),
+// 48 at N = 16 FP32 (P = 8, M = 6: 43 against 135 us) and 44 in FP64 (57
+// against 185 us).  So a split pays up to 5 or 6, 3 and 3 waves: at N = 24
+// 61 points take 1,011 us split, 74 points 1,210 us split and 90 or more
+// points, whole, 1,194 us; at N = 16 49 points take 130 us split and 61 or more,
+// whole, 135 us (FP64 170 and 185 us).  Only 1 or P chunks: with one node per
+// chunk the final sum over the chunks' slices adds the nodes in the same order
+// as the unsplit accumulation, so a point's Q does not depend on the launch it
+// is part of (bit for bit).  Items are capped at kCubeSlices per CTA of the grid
+// (the partial-spectrum scratch), and more points than CTAs are not split.
 // Every CTA computes the same value.
 __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
   if (P < 2 || npts > G || (long long)npts * P > (long long)kCubeSlices * G) return 1;
@@ -129,8 +131,10 @@ __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
 
 // Cycles between the starts of the second pass of a scheduler's successive
 // warps: staggered, the loads of one warp run beside the arithmetic of
-// another and the stores of a third (4.20 ms against 4.38 ms per 576 points
-// at N = 24 without; 60, 100 and 200 cycles measure the same).
+// another and the stores of a third (N = 24, five warps per scheduler: 4.76 ms
+// per 576 points against 4.81 ms without; 60, 100 and 200 cycles measure the
+// same; at N = 16, two or three warps, with and without measure the same in
+// either precision, so it is left out there).
 constexpr unsigned kStagger = 100;
 
 template <typename T, int N, int MINB>
@@ -139,6 +143,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
   using C = vx<T>;   // in registers
   using CM = cx<T>;  // in the tables and the scratch
   constexpr int WD = G::WD;
+  constexpr bool ROT = sizeof(T) == 8;  // F^ = (1 + i) F, else F
   constexpr int HN = G::HN, NN = G::NN, V = G::V, NM = G::NM, GT = G::GT, NT = G::NT, PS = G::PS, PHS = G::PHS;
   constexpr int B_ALL = 0, B_T = 1, B_G = 2;  // named barriers: CTA, Nyquist tables, groups
 
@@ -177,7 +182,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
     C x[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) x[j] = w2p[G::off(j)];
-    cfft<N, S>(x);
+    vfft<N, S>(x);
 #pragma unroll
     for (int j = 0; j < N; ++j) w2p[G::off(j)] = x[j];
   };
@@ -200,9 +205,16 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       if (n < 3 * N) dst[n] = e[i];
       if (n < 3 * N && n % N == HN) {
         const CM ce = mk<CM>(e[i].x, -e[i].y);
-        dst[3 * N + n / N] = cmul(ce, ce);
+        dst[3 * N + n / N] = mul_r(ce, ce);
       }
     }
+  };
+  // F^ at (k1, k2, k3) from the work cube; FP32: k3 > N/2 from the conjugate
+  // mirror
+  auto Fat = [&](int i1, int i2, int i3) -> C {
+    if (ROT || i3 <= HN) return sW[i1 * PS + G::off(i2) + i3];
+    const C c = sW[(N - i1) % N * PS + G::off((N - i2) % N) + N - i3];
+    return vmk(cre(c), -cim(c));
   };
   const int npts = a.pcount ? min(a.npts, *a.pcount) : a.npts;
   // work item = (point, chunk of radial nodes); with KP > 1 each chunk's
@@ -259,13 +271,13 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       s_it[3] = pt % a.neles;
     }
 
-    // ---- F^ = (1 + i) FFT(f) / V ---------------------------------------------
+    // ---- F^ from FFT(f) / V ---------------------------------------------
     if (is_main) {
       const int64_t b0 = soa_ix(pt / a.neles, a.ldim, pt % a.neles, (int64_t)(k1 * N + k2) * N, V, a.soasz);
       C x[N];
 #pragma unroll
       for (int k = 0; k < N; ++k) x[k] = vmk(a.f[b0 + (int64_t)k * a.soasz], T(0));
-      cfft<N, -1>(x);
+      vfft<N, -1>(x);
 #pragma unroll
       for (int k = 0; k < N; ++k) w1p[k] = x[k];
     }
@@ -277,16 +289,16 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       C x[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
-      cfft<N, -1>(x);
+      vfft<N, -1>(x);
 #pragma unroll
-      for (int i = 0; i < N; ++i) w3p[i * PS] = vmul(mul_1i<1>(x[i]), vmk(iv, iv));
+      for (int i = 0; i < N; ++i) w3p[i * PS] = vmul(ROT ? mul_1i<1>(x[i]) : x[i], vmk(iv, iv));
     }
     __syncthreads();
     if (is_main) {
       uint32_t t[2 * N * WD];
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        const C v = w1p[i];
+        const C v = Fat(k1, k2, i);
         tm_put(t, 2 * i, cre(v));
         tm_put(t, 2 * i + 1, cim(v));
       }
@@ -296,9 +308,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
 #pragma unroll 1
       for (int t = tq; t < 3 * N * N; t += G::NQ) {
         const int k = t / (3 * N), line = t % (3 * N), which = line / N, j = line % N;
-        sN[t] = which == 0   ? sW[HN * PS + G::off(j) + k]
-                : which == 1 ? sW[j * PS + G::off(HN) + k]
-                             : sW[j * PS + G::off(k) + HN];
+        sN[t] = which == 0 ? Fat(HN, j, k) : which == 1 ? Fat(j, HN, k) : Fat(j, k, HN);
       }
       CM e[NPH];
       phase_fetch(s_it[0] * a.M, e);
@@ -321,28 +331,20 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           // then m = Re(A E3[k3])
           {
             const CM* ph = sPh + slot * PHS;
-            const CM E12 = cmul(ph[k1], ph[N + k2]);
-            CM Et = E12;
-            if (k1 == HN) Et = cmul(Et, ph[3 * N]);
-            if (k2 == HN) Et = cmul(Et, ph[3 * N + 1]);
-            const CM s0 = cadd(E12, Et), s3 = cadd(E12, cmul(Et, ph[3 * N + 2]));
+            const CM E12 = mul_r(ph[k1], ph[N + k2]);
+            const CM th1 = ph[3 * N], th2 = ph[3 * N + 1];
+            const CM t12 = k1 != HN ? th2 : k2 == HN ? mul_r(th1, th2) : th1;
+            const CM Et = k1 == HN || k2 == HN ? mul_r(E12, t12) : E12;
+            const CM s0 = cadd(E12, Et), s3 = cadd(E12, mul_s(Et, ph[3 * N + 2]));
             const CM A = mk<CM>(T(0.5) * (s0.x + s0.y), T(0.5) * (s0.y - s0.x));
             const CM A3 = mk<CM>(T(0.5) * (s3.x + s3.y), T(0.5) * (s3.y - s3.x));
             C x[N];
             load_line(x);
             // e3[N - k] = conj e3[k]
-#pragma unroll
-            for (int k = 0; k <= HN; ++k) {
-              const CM e = ph[2 * N + k];
-              const CM& Ak = k == HN ? A3 : A;
-              const T c = Ak.x * e.x, m = c - Ak.y * e.y;
-              x[k] = vmk(cre(x[k]) * m, cim(x[k]) * m);
-              if (k > 0 && k < HN) {
-                const T n = c + Ak.y * e.y;
-                x[N - k] = vmk(cre(x[N - k]) * n, cim(x[N - k]) * n);
-              }
-            }
-            cfft<N, 1>(x);
+            vfft_scaled<N, 1>(x, [&](int k) {
+              const CM e = ph[2 * N + (k <= HN ? k : N - k)];
+              return re_mul(k == HN ? A3 : A, k <= HN ? e : mk<CM>(e.x, -e.y));
+            });
             mbar_wait_bounded(&s_read, rphase ^ 1, a.err, &s_gave_up);  // the previous cube is read
 #pragma unroll
             for (int k = 0; k < N; ++k) w1p[k] = x[k];
@@ -350,16 +352,15 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           slot ^= 1;
           bar_arrive(B_T, NT);        // done with the Nyquist tables of the previous (p, q)
           bar_sync(B_G + grp, GT);    // this group's planes are complete
-          if constexpr (NM / 32 > 4) {
+          if constexpr (NM / 32 > 8) {
             const unsigned t0 = clock();
             while (clock() - t0 < (unsigned)(wid >> 2) * kStagger) {
             }
           }
           pass2(std::integral_constant<int, 1>{});
           bar_sync(B_ALL, NT);        // the cube and the Nyquist tables are complete
-          // pass 3: lines (x2, x3) along k1; S += Re P Im P + Re Nq Im Nq with
+          // pass 3: lines (x2, x3) along k1; S += Re R^2 + Re Nq^2 with
           // Nq = s1 T1(x2, x3) + s2 T2(x1, x3) + s3 T3(x1, x2), s = (-1)^x
-          // (a common sign of Nq drops out: s3 Nq is formed)
           C x[N];
 #pragma unroll
           for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
@@ -369,21 +370,19 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           uint32_t t[N * WD];
           tmem_store_wait();
           tm_load(tmS, t);
-          cfft<N, 1>(x);
-          const T s3 = (x3 & 1) ? T(-1) : T(1), s23 = (x2 & 1) ? -s3 : s3;
-          const C t1 = vmul(sT1[x2 * N + x3], vmk(s3, s3)), ss = vmk(s23, s23);
+          vfft<N, 1>(x);
+          const T s2 = (x2 & 1) ? T(-1) : T(1), s3 = (x3 & 1) ? T(-1) : T(1);
+          const C t1 = sT1[x2 * N + x3], t1n = vmul(t1, vmk(T(-1), T(-1))), c2 = vmk(s2, s2), c3 = vmk(s3, s3);
           tm_wait(t);
 #pragma unroll
           for (int i = 0; i < N; ++i) {
-            const C u = sT3[x2 * (N + 1) + i];
-            const C n = vfma(sT2[i * N + x3], ss, (i & 1) ? vsub(u, t1) : vadd(u, t1));
-            const T s0 = q == 0 ? T(0) : tm_get(t, i, T(0));
-            tm_put(t, i, fma(cre(x[i]), cim(x[i]), fma(cre(n), cim(n), s0)));
+            const C n = vfma(sT3[x2 * (N + 1) + i], c3, vfma(sT2[i * N + x3], c2, (i & 1) ? t1n : t1));
+            tm_put(t, i, add_squares(x[i], n, q == 0 ? T(0) : tm_get(t, i, T(0))));
           }
           tm_store(tmS, t);
         }
         // FFT(S_p): lines of the third pass along x1 from the accumulators,
-        // each thread to the entries it read last, then planes k1 <= N/2
+        // each thread to the entries it read last, then planes k1 < GK
         {
           C x[N];
           tmem_store_wait();
@@ -392,14 +391,14 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           tm_wait(t);
 #pragma unroll
           for (int i = 0; i < N; ++i) x[i] = vmk(tm_get(t, i, T(0)), T(0));
-          cfft<N, -1>(x);
+          vfft<N, -1>(x);
 #pragma unroll
-          for (int i = 0; i <= HN; ++i) w3p[i * PS] = x[i];
+          for (int i = 0; i < G::GK; ++i) w3p[i * PS] = x[i];
         }
         bar_sync(B_ALL, NT);
-        if (k1 <= HN) pass2(std::integral_constant<int, -1>{});
+        if (k1 < G::GK) pass2(std::integral_constant<int, -1>{});
         bar_sync(B_ALL, NT);
-        if (k1 <= HN) {
+        if (k1 < G::GK) {
           // line (k1, k2) along x3.  All loads of the accumulated line are
           // issued before its first store (the slices could alias w1 as far
           // as the compiler knows)
@@ -408,7 +407,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           C x[N];
 #pragma unroll
           for (int k = 0; k < N; ++k) x[k] = w1p[k];
-          cfft<N, -1>(x);
+          vfft<N, -1>(x);
 #pragma unroll
           for (int k = 0; k < N; ++k) {
             const T w = __ldg(w1 + k * NN);
@@ -443,26 +442,19 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
             const bool p3 = which == 2;
             const CM* ph = sPh + slot * PHS;
             const CM th1 = ph[3 * N], th2 = ph[3 * N + 1], th3 = ph[3 * N + 2];
-            const CM Eb = cmul(ph[which == 0 ? HN : j], ph[which == 0 ? N + j : p3 ? 2 * N + HN : N + HN]);
-            CM tb = which == 0 ? th1 : p3 ? th3 : th2;
-            if (which == 0 && j == HN) tb = cmul(tb, th2);
-            const CM tb3 = cmul(tb, th3);
-            CM B = cmul(Eb, mk<CM>(T(1) - tb.x, -tb.y));
-            CM B3 = p3 ? mk<CM>(T(0), T(0)) : cmul(Eb, mk<CM>(T(1) - tb3.x, -tb3.y));
+            const CM Eb = mul_r(ph[which == 0 ? HN : j], ph[which == 0 ? N + j : p3 ? 2 * N + HN : N + HN]);
+            const CM tb = p3 ? th3 : which == 1 ? th2 : j == HN ? mul_r(th1, th2) : th1;
+            const CM tb3 = mul_r(tb, th3);
+            CM B = mul_1m(Eb, tb);
+            CM B3 = p3 ? mk<CM>(T(0), T(0)) : mul_1m(Eb, tb3);
             if (which != 0 && j == HN) B = B3 = mk<CM>(T(0), T(0));
             const CM A = mk<CM>(T(0.5) * (B.x + B.y), T(0.5) * (B.y - B.x));
             const CM A3 = mk<CM>(T(0.5) * (B3.x + B3.y), T(0.5) * (B3.y - B3.x));
             const CM* ev = ph + (p3 ? N : 2 * N);
             C x[N];
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-              const C v = sN[k * 3 * N + line];
-              const CM e = ev[k];
-              const CM& Ak = k == HN ? A3 : A;
-              const T n = Ak.x * e.x - Ak.y * e.y;
-              x[k] = vmk(cre(v) * n, cim(v) * n);
-            }
-            cfft<N, 1>(x);
+            for (int k = 0; k < N; ++k) x[k] = sN[k * 3 * N + line];
+            vfft_scaled<N, 1>(x, [&](int k) { return re_mul(k == HN ? A3 : A, ev[k]); });
 #pragma unroll
             for (int k = 0; k < N; ++k) sX[line * (N + 1) + k] = x[k];
           }
@@ -475,7 +467,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
             C x[N];
 #pragma unroll
             for (int i = 0; i < N; ++i) x[i] = sX[(which * N + i) * (N + 1) + j];
-            cfft<N, 1>(x);
+            vfft<N, 1>(x);
             // element i of the column: T1[i][j], T2[i][j], T3[j][i]
             C* const d = which == 0 ? sT1 + j : which == 1 ? sT2 + j : sT3 + j * (N + 1);
             const int de = which == 2 ? 1 : N;
@@ -503,8 +495,8 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
     // Two transforms: fC, summed from FP32 transforms, carries round-off, and
     // packing it with b2 F into one transform would leak that round-off into
     // the loss term as a constant times f (a momentum error proportional to
-    // rho u).  The transform of b2 F^ gives (1 + i) times the real collision
-    // frequency: its real part, kept where S was.
+    // rho u).  Of the transform of b2 F^ (in FP64 (1 + i) times the real collision
+    // frequency) the real part is kept where S was.
     if (is_main) {
       const T* b2 = a.b2t + k1 * N + k2;
       C x[N];
@@ -514,7 +506,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
         const T b = __ldg(b2 + k * NN);
         x[k] = vmul(x[k], vmk(b, b));
       }
-      cfft<N, 1>(x);
+      vfft<N, 1>(x);
 #pragma unroll
       for (int k = 0; k < N; ++k) w1p[k] = x[k];
     }
@@ -525,7 +517,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       C x[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
-      cfft<N, 1>(x);
+      vfft<N, 1>(x);
       uint32_t t[N * WD];
 #pragma unroll
       for (int i = 0; i < N; ++i) tm_put(t, i, cre(x[i]));
@@ -534,10 +526,10 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
     }
     __syncthreads();
     // QG = Re IFFT(fC); the chunks' slices are summed in a fixed order (L2
-    // reads: other CTAs wrote them).  Planes k1 > N/2 are the conjugate
-    // mirror of k1 < N/2.
+    // reads: other CTAs wrote them).  FP64: planes k1 > N/2 are the
+    // conjugate mirror of k1 < N/2.
     if (is_main) {
-      const bool mir = k1 > HN;
+      const bool mir = k1 >= G::GK;
       const int line = mir ? (N - k1) * N + (N - k2) % N : k1 * N + k2;
       const int kp = s_kp, i0 = item - item % kp;
       const CM* src = (kp == 1 ? fcg : a.fcp + (size_t)i0 * G::SL) + line;
@@ -561,7 +553,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
         x[0] = vmk(cre(x[0]), -cim(x[0]));
         x[HN] = vmk(cre(x[HN]), -cim(x[HN]));
       }
-      cfft<N, 1>(x);
+      vfft<N, 1>(x);
 #pragma unroll
       for (int k = 0; k < N; ++k) w1p[k] = x[k];
     }
@@ -576,7 +568,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       C x[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = w3p[i * PS];
-      cfft<N, 1>(x);
+      vfft<N, 1>(x);
       sfor<0, N / SC>([&](auto cc) {
         constexpr int c = decltype(cc)::value;
         uint32_t t[SC * WD];

@@ -2,18 +2,19 @@
 // shared memory: FP32 at N = 32 and FP64 at N = 24.
 //
 // The same exact restatement of the reference's operator as the single-CTA
-// kernel (vhs_cube.cuh: one complex transform P = IFFT(m F^) per (p, q) with
-// F^ = (1 + i) F, the Nyquist-plane term Nq as three 2D transforms, Re S =
-// Re P Im P + Re Nq Im Nq, fC = sum_p w1_p FFT(S_p), Q = prefac (Re IFFT(fC) -
-// f Re IFFT(b2 F)); frfs/solvers/dgfs/scattering.py:227-286 and
+// kernel (vhs_cube.cuh: one complex transform IFFT(m F^) per (p, q), F^ =
+// (1 + i) F in FP64 and F in FP32, the Nyquist-plane term Nq as three 2D
+// transforms, Re S = Re R^2 + Re Nq^2, fC = sum_p w1_p FFT(S_p), Q = prefac
+// (Re IFFT(fC) - f Re IFFT(b2 F)); frfs/solvers/dgfs/scattering.py:227-286 and
 // vhs-gll.mako:103-266), for a thread-block cluster of two CTAs per solution
 // point, persistent over the bank.
 //
 // Data distribution (rank r of the pair, MH = N/2, Q = N/4):
 //   k-slab   CTA r owns MH planes k1, closed under k1 -> -k1 mod N, in slots
 //            (pair_kmap): K_0 = {0..Q-1, MH, N-Q+1..N-1}, K_1 = {Q..MH-1,
-//            MH+1..N-Q}; slots below Q (and slot Q of K_0, k1 = MH) hold the
-//            k1 <= N/2 the gain spectrum is kept for (S_p is real);
+//            MH+1..N-Q}; in FP64 slots below Q (and slot Q of K_0, k1 = MH) hold the
+//            k1 <= N/2 the gain spectrum is kept for (S_p is real), in FP32 it is
+//            kept on all lines for k3 <= N/2;
 //   x-slab   CTA r owns x2 in X_r = [MH r, MH r + MH).
 // A 3D inverse transform runs along k3 on the lines (k1 in K_r, k2), along
 // k2 on the lines (k1 in K_r, x3), then along k1 on the lines (x2 in X_r,
@@ -36,14 +37,16 @@
 // a warp is one plane k1, so the first two passes need no barrier at all
 // between them (N = 24: groups of 4 planes, 3 warps).  The third pass releases
 // the work cube as soon as its values are in registers.  NQ more threads
-// transform the Nyquist planes (one line each).  The Nyquist products, which
-// need only the CTA's own tables, are added while the halves travel.
-// Measured on one B200: FP32 N = 32 (16 x 24 (p, q)), 2,592 points: 109.9 ms a
-// sweep against 140.5 ms for the scalar-transform form (112.4 ms with the
-// Nyquist products after the third pass, 113.6 ms with the Nyquist lines on
-// main threads); FP64 N = 24, 576 points: 10.53 ms against 15.05 ms (10.98,
-// 11.82 ms).  Handing over by one thread's cluster-scope mbarrier arrivals after
-// a CTA barrier, instead of the cluster barrier, measured 120.4 and 11.79 ms.
+// transform the Nyquist planes (one line each).  In FP64 the Nyquist products,
+// which need only the CTA's own tables, are added while the halves travel; FP32
+// adds them after the third pass, in the order of roundings of fft_vec.cuh.
+// Measured on one B200: FP32 N = 32 (16 x 24 (p, q)), 2,592 points: 114.3 ms a
+// sweep against 140.5 ms for two lines per thread with scalar transforms, the
+// same values bit for bit (120.6 ms with the Nyquist lines on main threads);
+// FP64 N = 24, 576 points: 10.5 ms against 15.05 ms (11.8 ms; 10.98 ms with the
+// Nyquist products after the third pass).  Handing over by one thread's
+// cluster-scope mbarrier arrivals after a CTA barrier, instead of the cluster
+// barrier, was 7 to 8 % slower in either.
 //
 // Shared memory (complex): W [MH][N][N + 1], the Nyquist planes T1 [x2 in
 // X_r][x3], T2 [x1][x3], T3 [x2 in X_r][x1], F^ on them [k][line] and their
@@ -83,8 +86,11 @@ template <typename T, int N_, bool OWN> struct PairGeom {
   static constexpr int OFF_PH = OFF_X + 3 * N * LP;      // [2][PHS]
   static constexpr int SMEM = (OFF_PH + 2 * PHS) * 2 * (int)sizeof(T);  // bytes
   static constexpr int SLICE = H * NN;                   // F in the scratch, [k3][k1][k2]
-  static constexpr int GL = (Q + 1) * N;                 // gain spectrum lines per CTA
-  static constexpr int GSL = GL * N;                     // ... entries, [k3][line]
+  // gain spectrum of a CTA: FP64 the lines k1 <= N/2, FP32 every line for
+  // k3 <= N/2; the rest is the conjugate mirror
+  static constexpr int GL = sizeof(T) == 4 ? NM : (Q + 1) * N;  // lines
+  static constexpr int GK = sizeof(T) == 4 ? H : N;             // entries of a line
+  static constexpr int GSL = GL * GK;                           // [k3][line]
   static constexpr int XSLAB = MH * MH * N;              // entries per staging buffer [slot][j][x3]
   // scratch per pair: F, the gain spectra of both CTAs (which double as the
   // exchange buffer of the forward transform of f), [2 CTAs][2] staging
@@ -118,6 +124,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
   using CM = cx<T>;  // in the tables and the scratch
   constexpr int N = G::N, NY = G::NY, NN = G::NN, V = G::V, LP = G::LP, NM = G::NM, MH = G::MH, Q = G::Q;
   constexpr int NT = G::NT, GT = G::GT, PHS = G::PHS, WD = G::WD;
+  constexpr bool ROT = sizeof(T) == 8;  // F^ = (1 + i) F, else F
   constexpr int B_T = 1, B_N = 2, B_G = 3;  // named barriers: old and new Nyquist tables, groups
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -154,7 +161,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
   C* const w1p = sW + tid * LP;                // line (slot, k2) along k3
   C* const w2p = sW + hi * N * LP + lo;        // line (slot, x3) along k2: stride LP
   C* const w3p = sW + x2 * LP + lo;            // line (x2, x3) along the slots: stride N LP
-  const bool gain_line = hi < Q || (hi == Q && r == 0);  // k1 <= N/2
+  const bool gain_line = !ROT || hi < Q || (hi == Q && r == 0);  // FP64: k1 <= N/2
   uint32_t peer = (uint32_t)(r ^ 1);
   int xb = 0;  // staging buffer of the next exchange
   auto xmine = [&]() { return Xs + (size_t)(r * 2 + xb) * G::XSLAB + lo; };
@@ -190,7 +197,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
     C x[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) x[j] = w2p[j * LP];
-    cfft<N, +1>(x);
+    vfft<N, +1>(x);
     CM* const xs = xmine() + hi * MH * N;
 #pragma unroll
     for (int j = 0; j < MH; ++j) {
@@ -218,7 +225,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       dst[tq] = e;
       if (tq % N == NY) {
         const CM ce = mk<CM>(e.x, -e.y);
-        dst[3 * N + tq / N] = cmul(ce, ce);
+        dst[3 * N + tq / N] = mul_r(ce, ce);
       }
     }
   };
@@ -232,26 +239,19 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
     if (tq < 3 * N) {
       const CM* ph = sPh + slot * PHS;
       const CM th1 = ph[3 * N], th2 = ph[3 * N + 1], th3 = ph[3 * N + 2];
-      const CM Eb = cmul(ph[which == 0 ? NY : jn], ph[which == 0 ? N + jn : p3 ? 2 * N + NY : N + NY]);
-      CM tb = which == 0 ? th1 : p3 ? th3 : th2;
-      if (which == 0 && jn == NY) tb = cmul(tb, th2);
-      const CM tb3 = cmul(tb, th3);
-      CM B = cmul(Eb, mk<CM>(T(1) - tb.x, -tb.y));
-      CM B3 = p3 ? mk<CM>(T(0), T(0)) : cmul(Eb, mk<CM>(T(1) - tb3.x, -tb3.y));
+      const CM Eb = mul_r(ph[which == 0 ? NY : jn], ph[which == 0 ? N + jn : p3 ? 2 * N + NY : N + NY]);
+      const CM tb = p3 ? th3 : which == 1 ? th2 : jn == NY ? mul_r(th1, th2) : th1;
+      const CM tb3 = mul_r(tb, th3);
+      CM B = mul_1m(Eb, tb);
+      CM B3 = p3 ? mk<CM>(T(0), T(0)) : mul_1m(Eb, tb3);
       if (which != 0 && jn == NY) B = B3 = mk<CM>(T(0), T(0));
       const CM A = mk<CM>(T(0.5) * (B.x + B.y), T(0.5) * (B.y - B.x));
       const CM A3 = mk<CM>(T(0.5) * (B3.x + B3.y), T(0.5) * (B3.y - B3.x));
       const CM* ev = ph + (p3 ? N : 2 * N);
       C x[N];
 #pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const C v = sN[k * 3 * N + tq];
-        const CM e = ev[k];
-        const CM& Ak = k == NY ? A3 : A;
-        const T n = Ak.x * e.x - Ak.y * e.y;
-        x[k] = vmk(cre(v) * n, cim(v) * n);
-      }
-      cfft<N, 1>(x);
+      for (int k = 0; k < N; ++k) x[k] = sN[k * 3 * N + tq];
+      vfft_scaled<N, 1>(x, [&](int k) { return re_mul(k == NY ? A3 : A, ev[k]); });
 #pragma unroll
       for (int k = 0; k < N; ++k) sX[tq * LP + k] = x[k];
     }
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       C x[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = sX[(which * N + i) * LP + jn];
-      cfft<N, 1>(x);
+      vfft<N, 1>(x);
       if (which == 0) {  // rows x2 of this CTA's half
 #pragma unroll
         for (int i = 0; i < MH; ++i) sT1[i * N + jn] = r ? x[MH + i] : x[i];
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       C x[N];
 #pragma unroll
       for (int k = 0; k < N; ++k) x[k] = vmk(a.f[b0 + (int64_t)k * a.soasz], T(0));
-      cfft<N, -1>(x);
+      vfft<N, -1>(x);
 #pragma unroll
       for (int k = 0; k <= NY; ++k) w1p[k] = x[k];
     }
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       C x[N];
 #pragma unroll
       for (int j = 0; j < N; ++j) x[j] = sW[(x1l * N + j) * LP + k3];
-      cfft<N, -1>(x);
+      vfft<N, -1>(x);
 #pragma unroll
       for (int j = 0; j < N; ++j) Xf[(k3 * N + MH * r + x1l) * N + j] = to_c(x[j]);
     }
@@ -316,17 +316,18 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       C x[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = from_c(__ldcg(Xf + (k3 * N + i) * N + k2));
-      cfft<N, -1>(x);
+      vfft<N, -1>(x);
 #pragma unroll
       for (int i = 0; i < N; ++i) Fg[(k3 * N + i) * N + k2] = to_c(vmul(x[i], vmk(iv, iv)));
     }
     cl_sync();  // F complete in the scratch; the exchange buffer may be reused
-    // F^ = (1 + i) F at (k1, k2, k3) from the half spectrum (written by both
-    // CTAs: read through L2)
+    // F^ at (k1, k2, k3) from the half spectrum (written by both CTAs:
+    // read through L2)
     auto Fat = [&](int i1, int i2, int i3) -> C {
-      if (i3 <= NY) return mul_1i<1>(from_c(__ldcg(Fg + (i3 * N + i1) * N + i2)));
-      const CM c = __ldcg(Fg + ((N - i3) * N + (N - i1) % N) * N + (N - i2) % N);
-      return mul_1i<1>(vmk(c.x, -c.y));
+      const bool mir = i3 > NY;
+      const CM c = __ldcg(Fg + (mir ? ((N - i3) * N + (N - i1) % N) * N + (N - i2) % N : (i3 * N + i1) * N + i2));
+      const C v = vmk(c.x, mir ? -c.y : c.y);
+      return ROT ? mul_1i<1>(v) : v;
     };
     if (is_main) {
       uint32_t t[2 * N * WD];
@@ -368,28 +369,20 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           // pass 1: m F^ along k3 (vhs_cube.cuh)
           {
             const CM* ph = sPh + slot * PHS;
-            const CM E12 = cmul(ph[k1], ph[N + lo]);
-            CM Et = E12;
-            if (k1 == NY) Et = cmul(Et, ph[3 * N]);
-            if (lo == NY) Et = cmul(Et, ph[3 * N + 1]);
-            const CM s0 = cadd(E12, Et), s3 = cadd(E12, cmul(Et, ph[3 * N + 2]));
+            const CM E12 = mul_r(ph[k1], ph[N + lo]);
+            const CM th1 = ph[3 * N], th2 = ph[3 * N + 1];
+            const CM t12 = k1 != NY ? th2 : lo == NY ? mul_r(th1, th2) : th1;
+            const CM Et = k1 == NY || lo == NY ? mul_r(E12, t12) : E12;
+            const CM s0 = cadd(E12, Et), s3 = cadd(E12, mul_s(Et, ph[3 * N + 2]));
             const CM A = mk<CM>(T(0.5) * (s0.x + s0.y), T(0.5) * (s0.y - s0.x));
             const CM A3 = mk<CM>(T(0.5) * (s3.x + s3.y), T(0.5) * (s3.y - s3.x));
             C x[N];
             load_line(x);
             // e3[N - k] = conj e3[k]
-#pragma unroll
-            for (int k = 0; k <= NY; ++k) {
-              const CM e = ph[2 * N + k];
-              const CM& Ak = k == NY ? A3 : A;
-              const T c = Ak.x * e.x, m = c - Ak.y * e.y;
-              x[k] = vmk(cre(x[k]) * m, cim(x[k]) * m);
-              if (k > 0 && k < NY) {
-                const T n = c + Ak.y * e.y;
-                x[N - k] = vmk(cre(x[N - k]) * n, cim(x[N - k]) * n);
-              }
-            }
-            cfft<N, 1>(x);
+            vfft_scaled<N, 1>(x, [&](int k) {
+              const CM e = ph[2 * N + (k <= NY ? k : N - k)];
+              return re_mul(k == NY ? A3 : A, k <= NY ? e : mk<CM>(e.x, -e.y));
+            });
             mbar_wait_bounded(&s_read, rphase ^ 1, a.err, &s_gave_up);  // the previous cube is read
 #pragma unroll
             for (int k = 0; k < N; ++k) w1p[k] = x[k];
@@ -405,54 +398,49 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           group_sync();
           pass2_out();
           cl_arrive();
-          // While the halves travel: S += Re Nq Im Nq on this thread's
-          // third-pass line, Nq = s1 T1(x2, x3) + s2 T2(x1, x3) + s3 T3(x1, x2)
-          // with s = (-1)^x (a common sign drops out: s3 Nq is formed)
+          // S += Re R^2 + Re Nq^2 on this thread's third-pass line, Nq = s1 T1(x2,
+          // x3) + s2 T2(x1, x3) + s3 T3(x1, x2) with s = (-1)^x.  FP64 adds
+          // Re Nq^2 while the halves travel; FP32 both at once after the third
+          // pass, in the order in which they are rounded
           bar_sync(B_N, NT);    // the Nyquist tables are complete
           constexpr int SC = 8;  // values per step
-          tmem_store_wait();
-          {
-            const T s3 = (lo & 1) ? T(-1) : T(1), s23 = (x2 & 1) ? -s3 : s3;
-            const C t1 = vmul(sT1[tid], vmk(s3, s3)), ss = vmk(s23, s23);
+          const T s2 = (x2 & 1) ? T(-1) : T(1), s3 = (lo & 1) ? T(-1) : T(1);
+          const C t1 = sT1[tid], t1n = vmul(t1, vmk(T(-1), T(-1))), c2 = vmk(s2, s2), c3 = vmk(s3, s3);
+          auto nyq_at = [&](int i) {
+            return vfma(sT3[hi * LP + i], c3, vfma(sT2[i * N + lo], c2, (i & 1) ? t1n : t1));
+          };
+          // S <- f(i, S) over the line
+          auto update = [&](auto&& f) {
+            tmem_store_wait();
             sfor<0, N / SC>([&](auto cc) {
               constexpr int c = decltype(cc)::value;
               uint32_t t[SC * WD];
               tm_load(tmS + SC * c * WD, t);
               tm_wait(t);
 #pragma unroll
-              for (int h = 0; h < SC; ++h) {
-                const int i = SC * c + h;
-                const C u = sT3[hi * LP + i];
-                const C n = vfma(sT2[i * N + lo], ss, (i & 1) ? vsub(u, t1) : vadd(u, t1));
-                tm_put(t, h, fma(cre(n), cim(n), q == 0 ? T(0) : tm_get(t, h, T(0))));
-              }
+              for (int h = 0; h < SC; ++h) tm_put(t, h, f(SC * c + h, tm_get(t, h, T(0))));
               tm_store(tmS + SC * c * WD, t);
+            });
+          };
+          if constexpr (ROT) {
+            update([&](int i, T s) {
+              const C n = nyq_at(i);
+              return fma(cre(n), cim(n), q == 0 ? T(0) : s);
             });
           }
           cl_wait();            // both halves staged
-          // pass 3: lines (x2, x3) along k1; S += Re P Im P
+          // pass 3: lines (x2, x3) along k1
           C x[N];
           load3(x);
           __syncwarp();
           if (tid % 32 == 0) mbar_arrive(&s_read);  // this warp's part of the cube may be overwritten
           rphase ^= 1;
-          cfft<N, 1>(x);
-          tmem_store_wait();
-          sfor<0, N / SC>([&](auto cc) {
-            constexpr int c = decltype(cc)::value;
-            uint32_t t[SC * WD];
-            tm_load(tmS + SC * c * WD, t);
-            tm_wait(t);
-#pragma unroll
-            for (int h = 0; h < SC; ++h) {
-              const C v = x[SC * c + h];
-              tm_put(t, h, fma(cre(v), cim(v), tm_get(t, h, T(0))));
-            }
-            tm_store(tmS + SC * c * WD, t);
-          });
+          vfft<N, 1>(x);
+          if constexpr (ROT) update([&](int i, T s) { return fma(cre(x[i]), cim(x[i]), s); });
+          else update([&](int i, T s) { return add_squares(x[i], nyq_at(i), q == 0 ? T(0) : s); });
         }
 
-        // fC += w1_p FFT(S_p) on the planes k1 <= N/2: lines (x2, x3) along x1
+        // fC += w1_p FFT(S_p) on the gain lines: lines (x2, x3) along x1
         // from S (each thread to the entries it read last), the exchange to
         // k-slabs, lines (k1, x3) along x2, lines (k1, k2) along x3
         {
@@ -463,10 +451,10 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           tm_wait(t);
 #pragma unroll
           for (int i = 0; i < N; ++i) x[i] = vmk(tm_get(t, i, T(0)), T(0));
-          cfft<N, -1>(x);
+          vfft<N, -1>(x);
           CM* const xs = xmine() + hi * N;
 #pragma unroll
-          for (int k = 0; k <= NY; ++k) {
+          for (int k = 0; k < (ROT ? NY + 1 : N); ++k) {
             if (pair_owner<N>(k) == r) w3p[pair_kinv<N>(k) * N * LP] = x[k];
             else __stcg(xs + pair_kinv<N>(k) * MH * N, to_c(x[k]));
           }
@@ -477,7 +465,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           C x[N];
 #pragma unroll
           for (int j = 0; j < N; ++j) x[j] = j / MH == r ? w2p[j * LP] : from_c(__ldcg(xp + (j % MH) * N));
-          cfft<N, -1>(x);
+          vfft<N, -1>(x);
 #pragma unroll
           for (int j = 0; j < N; ++j) w2p[j * LP] = x[j];
         }
@@ -489,18 +477,18 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
           C x[N];
 #pragma unroll
           for (int k = 0; k < N; ++k) x[k] = w1p[k];
-          cfft<N, -1>(x);
+          vfft<N, -1>(x);
           // read-modify-write in steps of 8: the loads of a step issued
           // together, fewer live registers than the whole line
 #pragma unroll
-          for (int k0 = 0; k0 < N; k0 += 8) {
+          for (int k0 = 0; k0 < G::GK; k0 += 8) {
             C acc[8];
             if (p > 0) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) acc[k] = from_c(fca[(k0 + k) * G::GL]);
+              for (int k = 0; k < 8 && k0 + k < G::GK; ++k) acc[k] = from_c(fca[(k0 + k) * G::GL]);
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 8 && k0 + k < G::GK; ++k) {
               const T w = __ldg(w1 + (k0 + k) * NN);
               const C v = vmul(x[k0 + k], vmk(w, w));
               fca[(k0 + k) * G::GL] = to_c(p > 0 ? vadd(acc[k], v) : v);
@@ -532,9 +520,9 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
 
     // ---- Q = prefac (Re IFFT(fC) - f Re IFFT(b2 F)) ----------------------------
     // Two inverse transforms: of b2 F^ (its real part, the collision
-    // frequency, kept where S was), then of the gain spectrum, whose planes
-    // k1 > N/2 are the conjugate mirror of k1 < N/2.  The staging buffer's
-    // index is a main thread's business; every thread takes the barriers.
+    // frequency, kept where S was), then of the gain spectrum.  The staging
+    // buffer's index is a main thread's business; every thread takes the
+    // barriers.
     double lam[5] = {0, 0, 0, 0, 0}, mom[5] = {0, 0, 0, 0, 0};
     // bank entries v = i N^2 + x2 N + x3 are b0 + i st
     const int64_t b0 = soa_ix(upt, a.ldim, elem, (int64_t)x2 * N + lo, V, a.soasz), st = (int64_t)NN * a.soasz;
@@ -551,16 +539,16 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
             x[k] = vmul(x[k], vmk(b, b));
           }
         } else {
-          const bool mir = !gain_line;
-          const int m1 = mir ? (N - k1) % N : k1, m2 = mir ? (N - lo) % N : lo;
-          const CM* const src = fC + pair_kinv<N>(m1) * N + m2;
+          const CM* const src = fC + tid;
+          const CM* const srm = fC + pair_kinv<N>((N - k1) % N) * N + (N - lo) % N;  // the mirrored line
 #pragma unroll
           for (int k = 0; k < N; ++k) {
-            const CM c = src[(mir ? (N - k) % N : k) * G::GL];
+            const bool mir = ROT ? !gain_line : k > NY;
+            const CM c = mir ? srm[(N - k) % N * G::GL] : src[k * G::GL];
             x[k] = vmk(c.x, mir ? -c.y : c.y);
           }
         }
-        cfft<N, 1>(x);
+        vfft<N, 1>(x);
 #pragma unroll
         for (int k = 0; k < N; ++k) w1p[k] = x[k];
         group_sync();
@@ -570,7 +558,7 @@ __global__ void __launch_bounds__(PairGeom<T, NV, OWN>::NT, 1) vhs_pair_kernel(c
       if (is_main) {
         C x[N];
         load3(x);
-        cfft<N, 1>(x);
+        vfft<N, 1>(x);
         constexpr int SC = 8;
         sfor<0, N / SC>([&](auto cc) {
           constexpr int c = decltype(cc)::value;

@@ -52,7 +52,7 @@ def sampled(Q):
     return Q[::{16: 1, 24: 5, 32: 11}[round(len(Q)**(1/3))]]
 
 
-@pytest.mark.parametrize('Nv', [16])
+@pytest.mark.parametrize('Nv', sorted(GRIDS))
 def test_values_keep_their_rounding(Nv):
     """To 5e-8 of the gain: transforms with other roundings give values 1.6e-7
     to 2.1e-7 away (FP32 round-off itself), a rare last bit far less."""
