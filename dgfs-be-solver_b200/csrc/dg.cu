@@ -49,12 +49,12 @@ constexpr int kDgNumShapes = sizeof(kDgShapes) / sizeof(kDgShapes[0]);
 // The shape a handle starts with: Runge-Kutta terms loaded ahead (every
 // measured mesh gains 10-25 %) and as many velocities per warp as leave enough
 // CTAs.  w = waves of 8-velocity CTAs; measured stage times in us with 8 / 4 / 2
-// velocities per warp: FP32 p = 2, 10 elements, N = 16 (w = 0.1) 55 / 44 / 41;
-// FP32 p = 2, 64 elements, N = 24 (1.0) 82.8 / 82.0 / 83.7; FP32 p = 3, 40
-// elements, N = 24 (1.5) 160 / 142 / 141; FP64 p = 2, 91 elements, N = 24 (2.2)
-// 182 / 173 / 180; FP64 p = 3, 64 elements, N = 24 (2.9) 213 / 226 / 248; FP32
-// p = 2, 288 elements, N = 32 (10) 552 / 553 / 598; FP32 p = 3, 640 elements,
-// N = 32 (35) 2187 / 2285 / 2335.
+// velocities per warp: FP32 p = 2, 10 elements, N = 16 (w = 0.1) 33 / 22 / 21;
+// FP32 p = 2, 64 elements, N = 24 (1.0) 71.9 / 71.4 / 71.8; FP32 p = 3, 40
+// elements, N = 24 (1.5) 130 / 115 / 121; FP64 p = 2, 91 elements, N = 24 (2.2)
+// 178 / 167 / 169; FP64 p = 3, 64 elements, N = 24 (2.9) 198 / 212 / 227; FP32
+// p = 2, 288 elements, N = 32 (10) 545 / 541 / 602; FP32 p = 3, 640 elements,
+// N = 32 (35) 2010 / 2055 / 2245.
 int default_shape(const dgfs_dg* h) {
   const int per_sm = h->prec == 32 ? (h->U <= 9 ? 3 : 2) : (h->U <= 9 ? 2 : 1);
   int sms = 148;
