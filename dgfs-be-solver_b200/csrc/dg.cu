@@ -46,7 +46,9 @@ struct DgShape {
 };
 constexpr DgShape kDgShapes[] = {{8, 0, 0}, {8, 1, 0}, {8, 1, 2}, {16, 1, 2}, {4, 0, 0}, {4, 1, 0}, {2, 1, 0}};
 constexpr int kDgNumShapes = sizeof(kDgShapes) / sizeof(kDgShapes[0]);
-// The shape a handle starts with: Runge-Kutta terms loaded ahead (every
+// The shape a handle starts with.  Matrices without 1D factors: the first one,
+// which adds the small Runge-Kutta terms first (the dense prefetching shapes
+// add them up ahead).  1D factors: Runge-Kutta terms loaded ahead (every
 // measured mesh gains 10-25 %) and as many velocities per warp as leave enough
 // CTAs.  w = waves of 8-velocity CTAs; measured stage times in us with 8 / 4 / 2
 // velocities per warp: FP32 p = 2, 10 elements, N = 16 (w = 0.1) 33 / 22 / 21;
@@ -56,6 +58,7 @@ constexpr int kDgNumShapes = sizeof(kDgShapes) / sizeof(kDgShapes[0]);
 // p = 2, 288 elements, N = 32 (10) 545 / 541 / 602; FP32 p = 3, 640 elements,
 // N = 32 (35) 2010 / 2055 / 2245.
 int default_shape(const dgfs_dg* h) {
+  if (!h->fac) return 0;
   const int per_sm = h->prec == 32 ? (h->U <= 9 ? 3 : 2) : (h->U <= 9 ? 2 : 1);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
@@ -358,15 +361,13 @@ template <typename T, int U, int F, int D, int VPT, int PF, int MB>
 cudaError_t launch_rhs(const dgfs_dg* h, const DgArgs<T>& a, int nv, cudaStream_t s) {
   constexpr int mb = MB ? MB : dg_default_mb<T, U, F, D>();
   constexpr int n = F / 4;
-  dim3 grid((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * VPT - 1) / (8 * VPT)));
+  const dim3 grid((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * VPT - 1) / (8 * VPT)));
   // with halo rows the face values of other partitions arrive by a
   // collective on another stream: the residual then waits in plain stream
   // order for everything before it
   if (h->fac)
     return launch_pdl(h->nhalo == 0, dg_residual_fac_kernel<T, n, VPT, PF, mb>, grid, s, a, make_fac<T, n>(h));
-  // matrices without 1D factors: one dense shape for every shape index
-  grid.y = (unsigned)((nv + 8 * kVpt - 1) / (8 * kVpt));
-  return launch_pdl(h->nhalo == 0, dg_residual_kernel<T, U, F, D, kVpt, 0, dg_default_mb<T, U, F, D>()>, grid, s, a,
+  return launch_pdl(h->nhalo == 0, dg_residual_kernel<T, U, F, D, VPT, PF, mb>, grid, s, a,
                     make_ops<T, U, F, D>(h));
 }
 

@@ -363,7 +363,7 @@ DGFS_API int dgfs_dg_invmass(dgfs_dg* h, const void* u, void* out, int v0,
  * index the velocities per warp, whether the Runge-Kutta terms are loaded
  * ahead of the flux work, and the CTAs per SM the register budget was
  * compiled for; dgfs_dg_select sets the shape of later dgfs_dg_rhs calls
- * (by default the one dgfs_dg_create picks for the mesh's size;
+ * (by default the one dgfs_dg_create picks for the operators and the size;
  * dgfs_dg_selected tells which).  No counterpart in the reference. */
 DGFS_API int dgfs_dg_num_variants(const dgfs_dg* h, int* count);
 DGFS_API int dgfs_dg_variant_info(const dgfs_dg* h, int idx, int* vpt,

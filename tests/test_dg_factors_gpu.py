@@ -36,6 +36,8 @@ def test_factored_and_dense_residual(precision, order, dense, monkeypatch):
     dg, sh, geo, vm = dg_setup(cfg, m)
     u = _states(vm, sh.nupts, geo.neles, seed=order)
     be, s = _system(cfg, m, u)
+    # without 1D factors a handle starts on the dense shape without prefetch
+    assert (s._dg_shape == 0) == (dense is not None)
     u_used = s.bank[0].get().astype(np.float64)
     uf = dg.disu(u_used)
     dg.update_bc(uf)
