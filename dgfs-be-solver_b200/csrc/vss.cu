@@ -328,10 +328,11 @@ void free_vss(dgfs_vss* h) {
 
 namespace {
 
-// [.][k3][k1 k2] -> [.][k1 k2][k3], one block per (direction, 32 lines)
+// [.][k3][k1 k2] -> [.][k1 k2][k3], one block per (direction, 32 lines); the
+// direction is the grid's x, whose extent has no limit of 65,535
 __global__ void untranspose_kernel(const float2* __restrict__ in, float2* __restrict__ out, int N) {
-  const int NN = N * N, l = blockIdx.x * 32 + threadIdx.x;
-  const size_t d = (size_t)blockIdx.y * NN * N;
+  const int NN = N * N, l = blockIdx.y * 32 + threadIdx.x;
+  const size_t d = (size_t)blockIdx.x * NN * N;
   if (l >= NN) return;
   for (int k = threadIdx.y; k < N; k += blockDim.y) out[d + (size_t)l * N + k] = in[d + (size_t)k * NN + l];
 }
@@ -344,17 +345,24 @@ int make_push_tables(dgfs_vss* h) {
     void** out;
     int dirs;
   } t[2] = {{h->bt, &h->b, h->P * h->M}, {h->bt_h, &h->b_h, h->P * h->Mh}};
+  // a table belongs to the handle once it is filled: a later call makes one
+  // that failed again
   for (auto& e : t) {
     if (!e.in || *e.out) continue;
-    if (cudaMalloc(e.out, (size_t)e.dirs * h->V * sizeof(float2)) != cudaSuccess) {
-      *e.out = nullptr;
+    void* table = nullptr;
+    if (cudaMalloc(&table, (size_t)e.dirs * h->V * sizeof(float2)) != cudaSuccess)
       return set_error(DGFS_ERR_NOMEM, "gain-kernel table allocation failed");
-    }
-    untranspose_kernel<<<dim3((h->N * h->N + 31) / 32, e.dirs), dim3(32, 8)>>>((const float2*)e.in, (float2*)*e.out,
+    cudaGetLastError();  // an earlier call's error is not this launch's
+    untranspose_kernel<<<dim3(e.dirs, (h->N * h->N + 31) / 32), dim3(32, 8)>>>((const float2*)e.in, (float2*)table,
                                                                                h->N);
+    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaDeviceSynchronize();
+    if (err != cudaSuccess) {
+      cudaFree(table);
+      return set_error(DGFS_ERR_CUDA, "gain-kernel tables: %s", cudaGetErrorString(err));
+    }
+    *e.out = table;
   }
-  if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
-    return set_error(DGFS_ERR_CUDA, "gain-kernel tables: %s", cudaGetErrorString(cudaGetLastError()));
   return DGFS_OK;
 }
 

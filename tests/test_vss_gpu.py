@@ -9,12 +9,15 @@ oracle (oracle/vss.py) restates the reference's operator in FP64.
 Tolerances (normwise relative, as the VHS tests): FP64 1e-10, FP32 2e-4.
 """
 
+import ctypes as ct
+
 import numpy as np
 import pytest
 import torch
 
 from conftest import SPHDESIGN
 from helpers import rel_err
+from frfs_b200 import _lib
 from frfs_b200.backend import B200Backend
 from frfs_b200.inifile import Inifile
 from frfs_b200.mixture import DGFSBiVelocityMesh, DGFSBiVSSGLLScatteringModel
@@ -23,6 +26,10 @@ from oracle import vss
 pytestmark = pytest.mark.gpu
 
 TOL = {'double': 1e-10, 'single': 2e-4}
+
+_lib.declare('dgfs_graph_begin', ct.c_int, [ct.c_void_p])
+_lib.declare('dgfs_graph_end', ct.c_int, [ct.c_void_p, ct.c_void_p])
+_lib.declare('dgfs_graph_destroy', ct.c_int, [ct.c_void_p])
 
 
 def mixture_config(precision, Nv=16, Nrho=6, M=12):
@@ -123,6 +130,38 @@ def test_vss_bank_matches_oracle(precision, Nv, pair):
             for s in range(2):
                 worst = max(worst, rel_err(got[s][u, :, e], Qo[s]))
     assert worst < TOL[precision], worst
+
+
+def test_select_after_a_refused_one():
+    """The cluster exchange kernel's tables are made when it is first
+    selected, which a stream capture refuses; the call after it makes them,
+    and the kernel agrees with the two-CTA one."""
+    cfg = mixture_config('single', Nv=24, Nrho=2)
+    be = B200Backend(cfg, device='cuda:0')
+    vm = DGFSBiVelocityMesh(be, cfg)
+    sm = DGFSBiVSSGLLScatteringModel(be, cfg, vm)
+    mesh, params, pre = _oracle(vm, cfg)
+    st = _states(mesh, 2, seed=24)
+    V = vm.vsize()
+    banks = [be.matrix((1, V, 2), np.array([x[s] for x in st]).T[None])
+             for s in range(2)]
+    ref, got = ([be.matrix((1, V, 2)) for _ in range(2)] for _ in range(2))
+    sm.fs_all(*banks, *ref)
+    lib, g = _lib.load(), ct.c_void_p()
+    side = torch.cuda.Stream(device=be.device)
+    torch.cuda.synchronize()
+    _lib.check(lib.dgfs_graph_begin(side.cuda_stream), 'dgfs_graph_begin')
+    try:
+        with pytest.raises(_lib.DgfsError):
+            sm.select(0)
+    finally:
+        lib.dgfs_graph_end(side.cuda_stream, ct.byref(g))
+        lib.dgfs_graph_destroy(g)
+    sm.select(0)
+    sm.fs_all(*banks, *got)
+    sm.status()
+    for r, o in zip(ref, got):
+        assert rel_err(o.get(), r.get()) < 2*TOL['single']
 
 
 def test_vss_single_point_leaves_the_rest():
