@@ -244,6 +244,10 @@ class MLP:
         self._cache = None
         self._sides = []
 
+    def __getstate__(self):
+        # copies and pickles take side streams of their own when they need them
+        return {**self.__dict__, '_sides': []}
+
     @property
     def _s(self):
         return torch.cuda.current_stream(self.device).cuda_stream

@@ -12,6 +12,9 @@ Tolerance: the products of BF16 operands are exact in FP32, so the only
 error is FP32 accumulation: 2e-5 of the largest output.
 """
 
+import copy
+import pickle
+
 import numpy as np
 import pytest
 import torch
@@ -256,3 +259,21 @@ def test_simt_tile_forms_agree(M, N, K, lay):
     cnt = torch.tensor([M], dtype=torch.int32, device=DEV)
     part = run(M + 40, cnt)
     assert torch.equal(part[:M], full[:M]) and torch.all(part[M:] == 7.0)
+
+
+@pytest.mark.parametrize('dup', [copy.deepcopy,
+                                 lambda m: pickle.loads(pickle.dumps(m))])
+def test_network_is_copied_after_a_training_step(dup):
+    """A network that has trained (and so holds streams) can be copied and
+    pickled; the copy computes the same and owns its memory."""
+    g = torch.Generator(device='cpu').manual_seed(3)
+    X, dY = (torch.randn(200, 256, generator=g).to(DEV) for _ in range(2))
+    mlp = surrogate.MLP(DEV, seed=3)
+    Y = mlp.forward(X, keep=True).clone()
+    G = {k: v.clone() for k, v in mlp.backward(dY).items()}
+    other = dup(mlp)
+    mlp.flat_w.zero_()
+    mlp.sync_bf16()
+    assert torch.equal(other.forward(X, keep=True), Y)
+    for k, v in other.backward(dY).items():
+        assert torch.equal(v, G[k])
