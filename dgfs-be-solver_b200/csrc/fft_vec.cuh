@@ -1,7 +1,9 @@
 // Register-resident complex FFTs of compile-time length, natural order in and
 // out, with the conventions of fft_reg.cuh:
 //
-//   cfft<N, S>(x):  x[k] <- sum_n x[n] exp(S 2 pi i n k / N)
+//   cfft<N, S>(x):  x[k] <- sum_n x[n] exp(S 2 pi i n k / N),  N = 8, 16, 24
+//   mfft<N, S>(x):  the same in FP32, N = 8, 16, 24, 32, with the roundings of
+//                   fft_reg.cuh (below)
 //
 // Two element types: double2, and cpx, an FP32 complex number in one 64-bit
 // register pair.  On cpx one packed instruction (add/sub/mul/fma.rn.f32x2)
@@ -13,8 +15,8 @@
 // adds (the same pipe time as one packed add) and the consumer is an FMA
 // with (-1, 1) factors.
 //
-// N = 2^m is a decimation in time down to 8-point kernels whose sqrt(1/2)
-// factors are folded into FMAs (52 operations).  N = 24 is the prime-factor
+// In cfft the 8-point kernels have their sqrt(1/2) factors folded into FMAs (52
+// operations), N = 16 is two of them and N = 24 the prime-factor
 // (Good-Thomas) transform: 3 and 8 have no common factor, so 8 three-point
 // and 3 eight-point transforms need no twiddle factors between them (252
 // operations against 308 for the mixed-radix 8 x 3 transform of fft_reg.cuh);
@@ -111,41 +113,28 @@ __device__ __forceinline__ double2 sub_half(double2 a, double2 b) {
   return make_double2(fma(b.x, -0.5, a.x), fma(b.y, -0.5, a.y));
 }
 // a + i S b
-template <int S> __device__ __forceinline__ cpx add_i(cpx a, cpx b) {
-  return S > 0 ? cpk(cre(a) - cim(b), cim(a) + cre(b)) : cpk(cre(a) + cim(b), cim(a) - cre(b));
-}
 template <int S> __device__ __forceinline__ double2 add_i(double2 a, double2 b) {
   return S > 0 ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, a.y - b.x);
 }
 // a (c + i s)
-__device__ __forceinline__ cpx mul_w(cpx a, double c, double s) {
-  const float wc = (float)c, ws = (float)s;
-  return cpk(fmaf(-ws, cim(a), wc * cre(a)), fmaf(ws, cre(a), wc * cim(a)));
-}
 __device__ __forceinline__ double2 mul_w(double2 a, double c, double s) {
   return make_double2(fma(-s, a.y, c * a.x), fma(s, a.x, c * a.y));
 }
 
-// cos(2 pi j / 32), j <= 8
-__host__ __device__ constexpr double cos32(int j) {
-  return j == 0 ? 1.0
-       : j == 1 ? 0.98078528040323044913
-       : j == 2 ? 0.92387953251128675613
-       : j == 3 ? 0.83146961230254523708
-       : j == 4 ? 0.70710678118654752440
-       : j == 5 ? 0.55557023301960222474
-       : j == 6 ? 0.38268343236508977173
-       : j == 7 ? 0.19509032201612826785
-                : 0.0;
+// cos(2 pi j / 96); sin(2 pi j / 96) = cos96(j - 24)
+__host__ __device__ constexpr double cos96(int j) {
+  constexpr double c[25] = {
+      1.0, 0.99785892323860350673, 0.99144486137381041114, 0.98078528040323044912, 0.96592582628906828674,
+      0.94693012949510566425, 0.92387953251128675612, 0.89687274153268830389, 0.86602540378443864676,
+      0.83146961230254523707, 0.79335334029123516457, 0.75183980747897739640, 0.70710678118654752440,
+      0.65934581510006886842, 0.60876142900872063941, 0.55557023301960222474, 0.5, 0.44228869021900128199,
+      0.38268343236508977172, 0.32143946530316158070, 0.25881904510252076234, 0.19509032201612826784,
+      0.13052619222005159154, 0.06540312923014306681, 0.0};
+  j = j < 0 ? -j : j;
+  j %= 96;
+  j = j > 48 ? 96 - j : j;
+  return j > 24 ? -c[48 - j] : c[j];
 }
-// cos and sin of 2 pi j / N (N divides 32), j < N / 2
-template <int N> __host__ __device__ constexpr double tcos(int j) {
-  return j * (32 / N) <= 8 ? cos32(j * (32 / N)) : -cos32(16 - j * (32 / N));
-}
-template <int N> __host__ __device__ constexpr double tsin(int j) {
-  return j * (32 / N) <= 8 ? cos32(8 - j * (32 / N)) : cos32(j * (32 / N) - 8);
-}
-
 // SW: the third output with its parts swapped
 template <int S, bool SW, typename C> __device__ __forceinline__ void cfft4(C& a, C& b, C& c, C& d) {
   const C s0 = vadd(a, c), d0 = vsub(a, c), s1 = vadd(b, d), d1 = sub_swap(b, d);
@@ -174,9 +163,8 @@ __device__ __forceinline__ void cfft8(C& x0, C& x1, C& x2, C& x3, C& x4, C& x5, 
 }
 
 template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[N]) {
-  if constexpr (N == 4) {
-    cfft4<S, false>(x[0], x[1], x[2], x[3]);
-  } else if constexpr (N == 8) {
+  static_assert(N == 8 || N == 16 || N == 24, "cfft lengths");
+  if constexpr (N == 8) {
     cfft8<S>(x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]);
   } else if constexpr (N == 24) {
     // n = 8 n1 + 3 n2, k = 16 k1 + 9 k2 (mod 24): W24^{nk} = W3^{n1 k1} W8^{n2 k2}
@@ -221,7 +209,7 @@ template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[
         x[j] = add_i<S>(e[j], o[j]);
         x[j + N / 2] = add_i<-S>(e[j], o[j]);
       } else {
-        const C t = j == 0 ? o[j] : mul_w(o[j], tcos<N>(j), S * tsin<N>(j));
+        const C t = j == 0 ? o[j] : mul_w(o[j], cos96(j * (96 / N)), S * cos96(j * (96 / N) - 24));
         x[j] = vadd(e[j], t);
         x[j + N / 2] = vsub(e[j], t);
       }
@@ -247,20 +235,6 @@ template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[
 //   mfft_scaled<N, S>(x, m): the same of x[k] m(k), real factors: the products
 //   of the first butterflies' leading terms are fused into their sums.
 
-// cos(2 pi j / 96), j <= 24
-__host__ __device__ constexpr double cos96(int j) {
-  constexpr double c[25] = {
-      1.0, 0.99785892323860350673, 0.99144486137381041114, 0.98078528040323044912, 0.96592582628906828674,
-      0.94693012949510566425, 0.92387953251128675612, 0.89687274153268830389, 0.86602540378443864676,
-      0.83146961230254523707, 0.79335334029123516457, 0.75183980747897739640, 0.70710678118654752440,
-      0.65934581510006886842, 0.60876142900872063941, 0.55557023301960222474, 0.5, 0.44228869021900128199,
-      0.38268343236508977172, 0.32143946530316158070, 0.25881904510252076234, 0.19509032201612826784,
-      0.13052619222005159154, 0.06540312923014306681, 0.0};
-  j = j < 0 ? -j : j;
-  j %= 96;
-  j = j > 48 ? 96 - j : j;
-  return j > 24 ? -c[48 - j] : c[j];
-}
 // i S a
 template <int S> __device__ __forceinline__ cpx rot_i(cpx a) {
   return S > 0 ? cpk(-cim(a), cre(a)) : cpk(cim(a), -cre(a));
@@ -386,8 +360,8 @@ template <int N, int S, typename M> __device__ __forceinline__ void vfft_scaled(
   }
   cfft<N, S>(x);
 }
-// a b, and a (1 - b), with the roundings of FP32 stated (which of the two
-// products is rounded by itself is the compiler's choice otherwise)
+// a b and a (1 - b) with the roundings of FP32 stated: which of the two products
+// of a sum is rounded by itself is the compiler's choice otherwise
 __device__ __forceinline__ float2 mul_r(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
 }
@@ -395,7 +369,7 @@ __device__ __forceinline__ float2 mul_1m(float2 a, float2 b) {
   const float c = 1.f - b.x;
   return make_float2(fmaf(a.y, b.y, __fmul_rn(a.x, c)), fmaf(a.y, c, -__fmul_rn(a.x, b.y)));
 }
-// a + a b, from ab: its imaginary part's other product is the rounded one
+// a b, the other product of the imaginary part rounded by itself
 __device__ __forceinline__ float2 mul_s(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
 }

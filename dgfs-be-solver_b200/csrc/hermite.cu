@@ -203,8 +203,9 @@ __device__ __forceinline__ void project_modes(const Field& g, int r, const Frame
 // the projection from there, and t1 then overlays the values.  576 points, N = 24,
 // FP32: 110 us (the L1's sectors 63 % busy) against 200 us with two passes over
 // the bank, a few loads in flight and 2.25 rows per thread.
-// STAGED = false (FP64 above N = 28, where the values do not fit): both read
-// the bank.
+// STAGED = false (FP64, where the values do not fit or cost more CTAs than they
+// save): both read the bank.  256 threads at least, for the contractions: N = 8,
+// 4 points 12.8 us, with 64 threads 16.6 us.
 template <typename T, bool STAGED, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) embed_kernel(const T* __restrict__ f, const T* __restrict__ Q,
                                                               const T* __restrict__ nu,
@@ -705,10 +706,13 @@ extern "C" int dgfs_hermite_embed(int precision, const void* f, const void* Q, c
   FrameArgs a{Nv, nupts, neles, ldim, L, cw, prefactor, gamma};
   const size_t vals = (size_t)Nv * Nv * Nv * (precision / 8), t1 = (size_t)(Nv * Nv + 1) * kP * sizeof(double),
                t2 = (size_t)Nv * kP * kP * sizeof(double);
-  // staged where the values fit beside 12 KB of tables (all of FP32, FP64 to N = 28)
-  const bool staged = std::max(vals, t1) + t2 <= (227 - 12) * 1024;
+  // staged where the values fit beside 12 KB of tables (all of FP32, FP64 to N =
+  // 28) unless they leave room for fewer CTAs of few warps (FP64 N = 16, 5,760
+  // points: 400 us staged, 361 us from the bank)
+  const bool staged =
+      std::max(vals, t1) + t2 <= (227 - 12) * 1024 && !(precision == 64 && Nv < 24 && vals > t1);
   const size_t smem = (staged ? std::max(vals, t1) : t1) + t2;
-  const unsigned grid = (unsigned)(nupts * neles), nt = (unsigned)((Nv * Nv + 31) / 32 * 32);
+  const unsigned grid = (unsigned)(nupts * neles), nt = (unsigned)std::max((Nv * Nv + 31) / 32 * 32, 256);
   auto launch = [&](auto* kernel, auto* fb) {
     using T = std::remove_pointer_t<decltype(fb)>;
     if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=

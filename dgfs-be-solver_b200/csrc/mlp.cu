@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(NTH, 2) gemm_kernel(int M, int N, int K, const
 // the 32 x 32 tiles.  With mcount, only the first *mcount rows exist: tiles past
 // it return at once.
 constexpr int FRM = 32, FRN = 8, FRK = 256, FRS = FRK + 4;  // FRS: lanes 4 banks apart
-constexpr int kRowsTiles = 148;
+constexpr int kRowsTiles = 148;  // one tile per SM
 static_assert(FRM * FRN == NTH, "one output per thread");
 
 template <typename TB>
