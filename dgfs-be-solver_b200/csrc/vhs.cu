@@ -119,11 +119,11 @@ template <typename T, int N, int C, int MINB> static VhsVariant make_push() {
 // Compiled launch shapes: (precision, N, cluster size, double-buffered
 // exchange, minimum CTAs per SM for the register budget).  The first entry
 // of each (precision, N) family is the default: the single-CTA kernel where a
-// point fits one SM (FP32 N = 24: 4.8 ms against 20 ms for the best cluster
+// point fits one SM (FP32 N = 24: 4.5 ms against 20 ms for the best cluster
 // shape on 576 points; FP64 N = 16: 59 us against 191 us on one point), else the
 // two-CTA kernel (FP64 N = 24: 11 ms against 50 ms on 576 points; FP32 N = 32:
 // 457 ms against 1,695 ms on 10,368).  FP32 N = 16 starts on the push kernel:
-// the single-CTA kernel takes 0.53 ms against 1.16 ms on 592 points, but its
+// the single-CTA kernel takes 0.48 ms against 1.16 ms on 592 points, but its
 // error against 64 bits is 1.2 times as large (up to 1.7 times on single
 // states); who wants it selects it.  The autotuner times the rest.
 static const std::vector<VhsVariant>& variants() {

@@ -59,11 +59,11 @@
 // threads transform the Nyquist planes and fetch the next phases.  The gain
 // spectrum is kept in a global (L2-resident) slice per CTA, [k3][line].
 //
-// Measured on one B200 (FP32, N = 24, 12 x 16 (p, q), 576 points): 4.76 ms a
+// Measured on one B200 (FP32, N = 24, 12 x 16 (p, q), 576 points): 4.54 ms a
 // sweep against 5.17 ms for two lines per thread with scalar transforms, with
 // the same roundings.  N = 16 (8 x 6): FP64, one point 59 us against 191 us for
 // the two-CTA push kernel (its radial nodes spread over the SMs); FP32, 592
-// points 0.53 ms against 1.16 ms, but its error is 1.2 times that of the push
+// points 0.48 ms against 1.16 ms, but its error is 1.2 times that of the push
 // kernel's two transforms per (p, q), so there it is not the default.
 #pragma once
 
@@ -109,20 +109,20 @@ template <typename T, int N> struct CubeGeom {
 // (3 M + 3) + kFixed) passes.  kFixed is what an item costs before its first
 // node and after its last (its own transform of f, the tables, the slice and
 // the point's last pass), fitted from the time per wave of split and of whole
-// items: 62 passes at N = 24 (P = 12, M = 16: 200 against 1,194 us a wave),
-// 48 at N = 16 FP32 (P = 8, M = 6: 43 against 135 us) and 44 in FP64 (57
-// against 185 us).  So a split pays up to 5 or 6, 3 and 3 waves: at N = 24
-// 61 points take 1,011 us split, 74 points 1,210 us split and 90 or more
-// points, whole, 1,194 us; at N = 16 49 points take 130 us split and 61 or more,
-// whole, 135 us (FP64 170 and 185 us).  Only 1 or P chunks: with one node per
-// chunk the final sum over the chunks' slices adds the nodes in the same order
-// as the unsplit accumulation, so a point's Q does not depend on the launch it
-// is part of (bit for bit).  Items are capped at kCubeSlices per CTA of the grid
-// (the partial-spectrum scratch), and more points than CTAs are not split.
+// items: 37 passes at N = 24 (P = 12, M = 16: 155 against 1,140 us a wave; M = 6:
+// 104 against 514 us), 47 at N = 16 FP32 (P = 8, M = 6: 39 against 123 us) and 44
+// in FP64 (57 against 185 us).  So a split pays up to 7, 3 and 3 waves, which 37
+// gives in all three: at N = 24 86 points take 1,086 us split and 87 or more,
+// whole, 1,140 us; at N = 16 55 points take 109 us split and 56 or more, whole,
+// 123 us (FP64 171 and 185 us).  Only 1 or P chunks: with one node per chunk the
+// final sum over the chunks' slices adds the nodes in the same order as the
+// unsplit accumulation, so a point's Q does not depend on the launch it is part
+// of (bit for bit).  Items are capped at kCubeSlices per CTA of the grid (the
+// partial-spectrum scratch), and more points than CTAs are not split.
 // Every CTA computes the same value.
 __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
   if (P < 2 || npts > G || (long long)npts * P > (long long)kCubeSlices * G) return 1;
-  constexpr double kFixed = 48.0;
+  constexpr double kFixed = 37.0;
   const double per_node = 3.0 * M + 3.0;
   const double whole = (double)((npts + G - 1) / G) * (P * per_node + kFixed);
   const double split = (double)(((long long)npts * P + G - 1) / G) * (per_node + kFixed);
@@ -131,8 +131,8 @@ __device__ __forceinline__ int cube_chunks(int npts, int G, int P, int M) {
 
 // Cycles between the starts of the second pass of a scheduler's successive
 // warps: staggered, the loads of one warp run beside the arithmetic of
-// another and the stores of a third (N = 24, five warps per scheduler: 4.76 ms
-// per 576 points against 4.81 ms without; 60, 100 and 200 cycles measure the
+// another and the stores of a third (N = 24, five warps per scheduler: 1 to 4 %
+// of a sweep; 60, 100 and 200 cycles measure the
 // same; at N = 16, two or three warps, with and without measure the same in
 // either precision, so it is left out there).
 constexpr unsigned kStagger = 100;
@@ -171,6 +171,11 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
   // roles of a main thread: first pass line (k1, k2), second pass line
   // (k1, x3 = r), third pass line (x2 = r, x3 = k1)
   const int grp = tid / GT, gu = tid % GT, k1 = 8 * grp + gu % 8, r = gu / 8, k2 = (r & 1) * HN + (r >> 1);
+  // place of line (k1, k2) in the gain spectrum: FP32, where only this thread
+  // touches it, by thread, so that a warp's accesses are whole 128-byte lines
+  // (N = 24: a point call 157 us, a sweep of 576 points 4.54 ms; by line 198 us
+  // and 4.76 ms, the sum of a split point's 12 slices alone 58 us); FP64 by line
+  const int gpos = G::GK == N ? tid : k1 * N + k2;
   C* const w1p = sW + k1 * PS + G::off(k2);
   C* const w2p = sW + k1 * PS + r;
   const int x2 = r, x3 = k1, wid = tid / 32;
@@ -403,7 +408,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
           // issued before its first store (the slices could alias w1 as far
           // as the compiler knows)
           const T* w1 = a.w1t + (size_t)p * V + k1 * N + k2;
-          CM* const fca = (s_kp == 1 ? fcg : a.fcp + (size_t)item * G::SL) + k1 * N + k2;
+          CM* const fca = (s_kp == 1 ? fcg : a.fcp + (size_t)item * G::SL) + gpos;
           C x[N];
 #pragma unroll
           for (int k = 0; k < N; ++k) x[k] = w1p[k];
@@ -530,9 +535,8 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
     // conjugate mirror of k1 < N/2.
     if (is_main) {
       const bool mir = k1 >= G::GK;
-      const int line = mir ? (N - k1) * N + (N - k2) % N : k1 * N + k2;
       const int kp = s_kp, i0 = item - item % kp;
-      const CM* src = (kp == 1 ? fcg : a.fcp + (size_t)i0 * G::SL) + line;
+      const CM* src = (kp == 1 ? fcg : a.fcp + (size_t)i0 * G::SL) + (mir ? (N - k1) * N + (N - k2) % N : gpos);
       C x[N];
 #pragma unroll
       for (int k = 0; k < N; ++k) x[k] = from_c(__ldcg(src + k * G::NL));
