@@ -40,6 +40,7 @@ All arithmetic runs in libdgfs_b200.so (embedding, gate, MLP forward and
 backward, Adam, reconstruction); PyTorch allocates the buffers.
 """
 
+import contextlib
 import ctypes as ct
 
 import numpy as np
@@ -292,9 +293,14 @@ class MLP:
                                  'ran out')
 
     def _fork(self, i):
-        """Side stream i of this network, behind the current stream: work
-        whose results the current stream needs only at the next join runs
-        beside it (as parallel branches when captured in a CUDA graph)."""
+        """Branch i of a captured step, behind the current stream: work whose
+        results the current stream needs only at the next join runs beside it
+        when the graph is replayed (batch 1,024: 131 us a step, 207 us as one
+        chain).  Outside a capture it stays on the current stream: a step is
+        then bound by its launches, and the forks and joins would double its
+        time (batch 128: 203 us, 407 us with them)."""
+        if not torch.cuda.is_current_stream_capturing():
+            return contextlib.nullcontext()
         cur = torch.cuda.current_stream(self.device)
         while len(self._sides) <= i:
             self._sides.append(torch.cuda.Stream(device=self.device))
@@ -302,6 +308,8 @@ class MLP:
         return torch.cuda.stream(self._sides[i])
 
     def _join(self, *sides):
+        if not torch.cuda.is_current_stream_capturing():
+            return
         cur = torch.cuda.current_stream(self.device)
         for i in sides:
             cur.wait_stream(self._sides[i])
@@ -556,14 +564,15 @@ class VHSSurrogate:
             b = self.ws._bufs[key] = self.backend.matrix(fbank.ioshape)
         return b
 
-    def loss_rate(self, fbank, nubank, gate=None):
-        """nu(c) at the points with gate != 0 (all when gate is None)."""
+    def loss_rate(self, fbank, nubank, gate=None, stream=None):
+        """nu(c) at the points with gate != 0 (all when gate is None), on the
+        raw stream (PyTorch's current one when None)."""
         nupts, _, neles = fbank.ioshape
         _, ldim, _ = fbank.traits
         _lib.check(_lib.load().dgfs_vhs_loss_rate(
             self.sm._h, fbank._as_parameter_, nubank._as_parameter_, nupts,
-            neles, ldim, self.backend.soasz, _p(gate), self._s),
-            'dgfs_vhs_loss_rate')
+            neles, ldim, self.backend.soasz, _p(gate),
+            self._s if stream is None else stream), 'dgfs_vhs_loss_rate')
         return nubank
 
     def embed(self, fbank, qbank=None, out=None, nubank=None):
@@ -763,6 +772,7 @@ class VHSSurrogate:
             self._side_nu = torch.cuda.Stream(device=self.device)
             self._fork = torch.cuda.Event()
             self._join = torch.cuda.Event()
+            self._join_nu = torch.cuda.Event()
         # made before the fork, on the stream whose memory pool it lives in
         nubank = self.nu_bank(fbank)
         self._fork.record(main)
@@ -775,11 +785,11 @@ class VHSSurrogate:
         # the collision frequency and the network (on the gate-1 rows only)
         # both need nothing but the gate: side by side
         self._side_nu.wait_event(self._fork)
-        with torch.cuda.stream(self._side_nu):
-            nu = self.loss_rate(fbank, nubank, gate)
+        nu = self.loss_rate(fbank, nubank, gate, self._side_nu.cuda_stream)
+        self._join_nu.record(self._side_nu)
         Bp = self.scale_targets(self.predict(X, net, nnet), eps,
                                 inverse=True)
-        main.wait_stream(self._side_nu)
+        main.wait_event(self._join_nu)
         work = ws.get('rwork', (nupts*(-(-neles//32))*32*(32*5 + NMODES),),
                       torch.float64)
         _lib.check(lib.dgfs_hermite_reconstruct(
