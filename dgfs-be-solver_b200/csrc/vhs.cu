@@ -874,10 +874,16 @@ cudaError_t launch_loss_rate(const dgfs_vhs* h, const void* f, void* nu, long lo
                              int soasz, const int* gate, cudaStream_t st) {
   const size_t smem = (size_t)N * N * (N / 2 + 1) * sizeof(cx<float>);
   // pairs where both spectra fit an SM (N <= 24) and two elements can be read at
-  // once: an even block size and stride, banks aligned to two values
+  // once: an even block size and stride, banks aligned to two values; and where
+  // there are more points than SMs: up to one point per SM nothing is shared and
+  // a pair takes longer (N = 24, FP32: 148 points 30.6 us singly, 39.8 us in
+  // pairs; 200 points 51.4 and 39.6 us; N = 16 12.5 and 14.5, 18.6 and 14.5 us)
   const size_t two = 2 * sizeof(TB);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
   if constexpr (N <= 24) {
-    if (soasz % 2 == 0 && ldim % 2 == 0 && (uintptr_t)f % two == 0 && (uintptr_t)nu % two == 0) {
+    if (neles > 1 && (long long)nupts * neles > sms && soasz % 2 == 0 && ldim % 2 == 0 && (uintptr_t)f % two == 0 &&
+        (uintptr_t)nu % two == 0) {
       const auto fn = loss_rate_pair_kernel<TB, N>;
       cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * smem));
       if (e != cudaSuccess) return e;

@@ -582,15 +582,20 @@ def test_loss_rate_of_neighbouring_elements(precision, Nv):
     sur = VHSSurrogate(sm)
     neles = 35
     f = random_states(vm.cv(), neles + 1, seed=Nv)
-    whole = _bank(be, f[None, :neles])
-    shifted = _bank(be, f[None, 1:])
-    a = sur.loss_rate(whole, be.matrix(whole.ioshape)).get()[0]
-    b = sur.loss_rate(shifted, be.matrix(shifted.ioshape)).get()[0]
-    assert np.array_equal(a[:, 1:], b[:, :-1])
-    gate = torch.zeros(neles, dtype=torch.int32, device=be.device)
+    # 35 points each have a CTA of their own; 175 share one in pairs (N <= 24)
+    alone = _bank(be, f[None, :neles])
+    whole = _bank(be, np.repeat(f[None, :neles], 5, 0))
+    shifted = _bank(be, np.repeat(f[None, 1:], 5, 0))
+    one, a, b = (sur.loss_rate(x, be.matrix(x.ioshape)).get()
+                 for x in (alone, whole, shifted))
+    for u in range(5):
+        assert np.array_equal(a[u], one[0])
+    assert np.array_equal(a[:, :, 1:], b[:, :, :-1])
+    gate = torch.zeros(5, neles, dtype=torch.int32, device=be.device)
     on = [0, 3, 6, 7, 34]
-    gate[on] = 1
+    gate[:, on] = 1
     out = be.matrix(whole.ioshape, np.full(whole.ioshape, 7.0))
-    c = sur.loss_rate(whole, out, gate).get()[0]
+    c = sur.loss_rate(whole, out, gate).get()
     off = [e for e in range(neles) if e not in on]
-    assert np.array_equal(c[:, on], a[:, on]) and np.all(c[:, off] == 7.0)
+    assert np.array_equal(c[:, :, on], a[:, :, on])
+    assert np.all(c[:, :, off] == 7.0)
