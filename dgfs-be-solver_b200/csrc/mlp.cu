@@ -15,6 +15,7 @@
 //                    device memory (dgfs_mlp_schedule writes them)
 //   dgfs_mlp_affine  y = (x - mu) * inv_sigma per column (and the inverse);
 //                    dgfs_mlp_affine_rows gathers / scatters through a row list
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -35,7 +36,7 @@ __device__ __forceinline__ float ld_b(const __nv_bfloat16* p) { return __bfloat1
 // round trips to L2 per output).
 template <int BM, int BN, int BK> constexpr int kTileFloats = BK * (BM + 4) + BK * (BN + 4);
 template <typename TB, int BM, int BN, int TM, int TN, int BK>
-__device__ __forceinline__ void gemm_tile(float* smem, int M, int N, int K, const float* __restrict__ A,
+__device__ __forceinline__ void gemm_tile(float* smem, int bx, int by, int M, int N, int K, const float* __restrict__ A,
                                           long long sam, long long sak, const TB* __restrict__ B, long long sbk,
                                           long long sbn, const float* __restrict__ bias, float* __restrict__ Z,
                                           float* __restrict__ C, long long ldc, int act, int accumulate) {
@@ -44,8 +45,8 @@ __device__ __forceinline__ void gemm_tile(float* smem, int M, int N, int K, cons
   float(*const Bs)[BN + 4] = reinterpret_cast<float(*)[BN + 4]>(smem + BK * (BM + 4));
   constexpr int TX = BN / TN;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  if (m0 >= M || n0 >= N) return;  // uniform over the CTA
+  const int m0 = by * BM, n0 = bx * BN;
+  if (m0 >= M) return;  // uniform over the CTA
   float acc[TM][TN] = {};
   // slices of K go through registers: every global load of a slice is
   // issued before any of its shared-memory stores, and the next slice's
@@ -118,13 +119,14 @@ __device__ __forceinline__ void gemm_tile(float* smem, int M, int N, int K, cons
 }
 
 template <typename TB, int BM, int BN, int TM, int TN, int BK>
-__global__ void __launch_bounds__(NTH, 2) gemm_kernel(int M, int N, int K, const float* __restrict__ A, long long sam,
+__global__ void __launch_bounds__(NTH, BM == 64 ? 3 : 2) gemm_kernel(int M, int N, int K, const float* __restrict__ A, long long sam,
                                                   long long sak, const TB* __restrict__ B, long long sbk,
                                                   long long sbn, const float* __restrict__ bias,
                                                   float* __restrict__ Z, float* __restrict__ C, long long ldc,
                                                   int act, int accumulate) {
   __shared__ __align__(16) float smem[kTileFloats<BM, BN, BK>];
-  gemm_tile<TB, BM, BN, TM, TN, BK>(smem, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate);
+  gemm_tile<TB, BM, BN, TM, TN, BK>(smem, blockIdx.x, blockIdx.y, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc,
+                                    act, accumulate);
 }
 
 // The same product, bit for bit (each sum runs over k in ascending order), for
@@ -153,12 +155,15 @@ __global__ void __launch_bounds__(NTH) gemm_rows_kernel(int M, const int* __rest
   static_assert(kTileFloats<32, 32, 64> <= (FRM + FRN) * FRS, "shared memory of both forms");
   float* const As = smem;              // [m][k]
   float* const Bs = smem + FRM * FRS;  // [n][k]
-  const int m0 = blockIdx.y * FRM, n0 = blockIdx.x * FRN;
   if (mcount) M = min(M, *mcount);
-  if ((long long)((M + FRM - 1) / FRM) * gridDim.x > max_tiles) {  // the grid covers these tiles too
-    gemm_tile<TB, 32, 32, 2, 2, 64>(smem, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate);
+  // the grid covers the tiles of either form
+  const int nf = (N + FRN - 1) / FRN, nt = (N + 31) / 32, bid = blockIdx.x;
+  if ((long long)((M + FRM - 1) / FRM) * nf > max_tiles) {
+    gemm_tile<TB, 32, 32, 2, 2, 64>(smem, bid % nt, bid / nt, M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act,
+                                    accumulate);
     return;
   }
+  const int m0 = bid / nf * FRM, n0 = bid % nf * FRN;
   if (m0 >= M) return;  // uniform over the CTA
   constexpr int LA = FRM * FRK / NTH, LB = FRN * FRK / NTH;
   float ra[LA], rb[LB];
@@ -389,12 +394,13 @@ static int gemm_pick(int M, const int* mcount, int N, int K, const float* A, lon
   // gemm_rows_kernel, which also takes the row counts only the device knows);
   // 32 x 32 tiles between.  The three give the same bits
   const long long tiles64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
-  const dim3 fr((N + FRN - 1) / FRN, (M + FRM - 1) / FRM);
+  const long long few = (long long)((N + FRN - 1) / FRN) * ((M + FRM - 1) / FRM);
+  const long long tiles32 = (long long)((N + 31) / 32) * ((M + 31) / 32);
   const int max_tiles = K > FRK / 2 ? kRowsTiles : 0;
   if (!mcount && tiles64 >= 148)
     gemm_launch<TB, 64, 64, 4, 4, 16>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
-  else if (mcount || (long long)fr.x * fr.y <= max_tiles)
-    gemm_rows_kernel<TB><<<fr, NTH, 0, s>>>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act,
+  else if (mcount || few <= max_tiles)
+    gemm_rows_kernel<TB><<<(unsigned)std::max(tiles32, std::min<long long>(few, max_tiles)), NTH, 0, s>>>(M, mcount, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act,
                                             accumulate, max_tiles);
   else
     gemm_launch<TB, 32, 32, 2, 2, 64>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Z, C, ldc, act, accumulate, s);
