@@ -64,13 +64,13 @@ struct FrameArgs {
   double L, cw, prefac, gamma;
 };
 
-__device__ __forceinline__ double block_sum(double v, double* red) {
+__device__ __forceinline__ double block_sum(double v, double* red, int warps) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   double s = 0;
-  for (int w = 0; w < (int)blockDim.x / 32; ++w) s += red[w];
+  for (int w = 0; w < warps; ++w) s += red[w];
   return s;
 }
 
@@ -99,8 +99,9 @@ __device__ __forceinline__ void point_frame(const Val& val, int r, const FrameAr
     s3 = tz;
     s4 = s0 * (cx * cx + cy * cy) + tzz;
   }
-  const double m0 = block_sum(s0, red), m1 = block_sum(s1, red), m2 = block_sum(s2, red),
-               m3 = block_sum(s3, red), m4 = block_sum(s4, red);
+  const int nw = blockDim.x / 32;
+  const double m0 = block_sum(s0, red, nw), m1 = block_sum(s1, red, nw), m2 = block_sum(s2, red, nw),
+               m3 = block_sum(s3, red, nw), m4 = block_sum(s4, red, nw);
   const double rho = m0 * a.cw, ux = m1 / m0, uy = m2 / m0, uz = m3 / m0;
   mom[0] = rho;
   mom[1] = ux;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(NT, MINB) embed_kernel(const T* __restrict__ f
     }
     X[(long long)pt * kFeat + k] = x;
   }
-  ne = block_sum(ne, red);
+  ne = block_sum(ne, red, blockDim.x / 32);
   if (threadIdx.x == 0) {
     eps[pt] = (float)sqrt(ne);
     for (int k = 0; k < 5; ++k) mom_out[(long long)pt * 5 + k] = mom[k];
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(kThreads) reconstruct_kernel(const float* __re
     // kernels: the point's slot in its AoSoA block)
     const long long slot = ((long long)upt * ((a.neles + 31) / 32) * 32 + e) * kRelaxSplit + chunk;  // chunk < kNetSplit
     for (int k = 0; k < 5; ++k) {
-      const double t = block_sum(mm[k], red);
+      const double t = block_sum(mm[k], red, kThreads / 32);
       if (threadIdx.x == 0) part[slot * 5 + k] = t;
     }
     return;
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(kThreads) reconstruct_kernel(const float* __re
   double lam[5];
   {
     double mt[5];
-    for (int k = 0; k < 5; ++k) mt[k] = block_sum(mm[k], red);
+    for (int k = 0; k < 5; ++k) mt[k] = block_sum(mm[k], red, kThreads / 32);
     for (int k = 0; k < 5; ++k) {
       double s = 0;
       for (int j = 0; j < 5; ++j) s += ginv[k * 5 + j] * mt[j];
