@@ -324,11 +324,6 @@ inline unsigned grid_for(const dgfs_dg* h, int nv) {
   return (unsigned)((nblk * nv * 32 + 255) / 256);
 }
 
-// (element block, velocity chunk of 8 * kVpt) grid of the interp/residual
-inline dim3 grid_blk(const dgfs_dg* h, int nv) {
-  return dim3((unsigned)((h->E + 31) / 32), (unsigned)((nv + 8 * kVpt - 1) / (8 * kVpt)));
-}
-
 template <typename T, int U, int F, int D>
 cudaError_t run_interp(const dgfs_dg* h, const void* u, int v0, int nv, cudaStream_t s) {
   DgArgs<T> a = make_args<T>(h);
