@@ -53,17 +53,17 @@ METRIC = 'Q(f) evals/s'
 # (kernel, workload, points, precision bits) -> (bytes, how it was taken)
 TRAFFIC = {
     ('vhs_cube_kernel', 'couette-n24', 576, 32):
-        (35.4e6, 'captured at this size'),
+        (40.1e6, 'captured at this size'),
     ('vhs_pair_kernel', 'channel-n32', 10368, 32):
-        (192.9e6*72, 'captured on the 4 x 4-element channel (144 points, '
-                     '192.9 MB, 608-thread layout) and scaled by the point '
+        (196.9e6*72, 'captured on the 4 x 4-element channel (144 points, '
+                     '196.9 MB, 608-thread layout) and scaled by the point '
                      'count (x72)'),
 }
 # the same for one DG stage (interp + residual): (workload, points, bits)
 DG_TRAFFIC = {
     ('couette-n24', 576, 32):
-        (190.1e6, 'captured at this size (interp 32.7 MB + residual '
-                  '157.4 MB, residual shape of 4 velocities per warp)'),
+        (188.4e6, 'captured at this size (interp 32.9 MB + residual '
+                  '155.5 MB, residual shape of 4 velocities per warp)'),
 }
 
 

@@ -226,10 +226,10 @@ template <int N, int S, typename C> __device__ __forceinline__ void cfft(C (&x)[
 // values: every sum, product and fused product is rounded where that
 // transform rounds it, so the results are its results bit for bit.  The
 // collision kernels take it in FP32 because Q near equilibrium is the small
-// difference of gain and loss (1e-4 of either at a distance of 1e-2) and shows
-// the transforms' round-off: with cfft above, whose N = 32 has two layers of
-// rounded twiddles, the error of Q rose by a factor 1.26 at N = 32; with cfft<24>
-// it fell by 0.78 at N = 24, but at a distance of 1e-2 either change is percents
+// difference of gain and loss (1e-6 to 1e-5 of either at a distance of 1e-2) and
+// shows the transforms' round-off: with two radix-2 layers of rounded twiddles
+// over 8-point kernels the error of Q was 1.26 times as large at N = 32; with
+// cfft<24> it is 0.78 times, but at a distance of 1e-2 either change is percents
 // of Q.
 //
 //   mfft_scaled<N, S>(x, m): the same of x[k] m(k), real factors: the products

@@ -295,7 +295,7 @@ class MLP:
     def _fork(self, i):
         """Branch i of a captured step, behind the current stream: work whose
         results the current stream needs only at the next join runs beside it
-        when the graph is replayed (batch 1,024: 131 us a step, 207 us as one
+        when the graph is replayed (batch 1,024: 114 us a step, 170 us as one
         chain).  Outside a capture it stays on the current stream: a step is
         then bound by its launches, and the forks and joins would double its
         time (batch 128: 203 us, 407 us with them)."""
@@ -544,8 +544,8 @@ class VHSSurrogate:
         self._last = None
         # the plain fallback runs on a few points: its own handle (it runs
         # on a side stream) with the single-CTA kernel, which splits few
-        # points into one work item per radial node (42 Couette points:
-        # 0.4 ms), else the cluster shape that spreads a point over the most
+        # points into one work item per radial node (49 Couette points:
+        # 0.62 ms), else the cluster shape that spreads a point over the most
         # SMs
         self._plain_h = (sm.make_handle('single-cta') or
                          sm.make_handle('push', largest_cluster=True) or sm._h)
