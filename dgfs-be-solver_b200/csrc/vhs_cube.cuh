@@ -506,12 +506,7 @@ __global__ void __launch_bounds__(CubeGeom<T, N>::NT, MINB) vhs_cube_kernel(cons
       const T* b2 = a.b2t + k1 * N + k2;
       C x[N];
       load_line(x);
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const T b = __ldg(b2 + k * NN);
-        x[k] = vmul(x[k], vmk(b, b));
-      }
-      vfft<N, 1>(x);
+      vfft_scaled<N, 1>(x, [&](int k) { return __ldg(b2 + k * NN); });
 #pragma unroll
       for (int k = 0; k < N; ++k) w1p[k] = x[k];
     }

@@ -41,8 +41,8 @@
 // which need only the CTA's own tables, are added while the halves travel; FP32
 // adds them after the third pass, in the order of roundings of fft_vec.cuh.
 // Measured on one B200: FP32 N = 32 (16 x 24 (p, q)), 2,592 points: 114.3 ms a
-// sweep against 140.5 ms for two lines per thread with scalar transforms, the
-// same values bit for bit (120.6 ms with the Nyquist lines on main threads);
+// sweep against 140.5 ms for two lines per thread with scalar transforms, with
+// the same roundings (120.6 ms with the Nyquist lines on main threads);
 // FP64 N = 24, 576 points: 10.5 ms against 15.05 ms (11.8 ms; 10.98 ms with the
 // Nyquist products after the third pass).  Handing over by one thread's
 // cluster-scope mbarrier arrivals after a CTA barrier, instead of the cluster
